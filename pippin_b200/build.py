@@ -14,13 +14,13 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIBDIR, "libpippin_b200.so")
-SOURCES = ["pg_kernels.cu", "pg_api.cpp", "pg_peak.cu", "pg_noalloc.cu", "pg_mlp.cu", "pg_render.cu"]
+SOURCES = ["pg_kernels.cu", "pg_lane.cu", "pg_quad.cu", "pg_api.cpp", "pg_peak.cu", "pg_noalloc.cu", "pg_mlp.cu", "pg_render.cu"]
 # the rasteriser rounds every product and sum on its own (no FMA contraction),
 # so that its coverage, depth and shading match an IEEE single-precision
 # evaluation of the same expressions on the CPU bit for bit
 EXTRA_FLAGS = {"pg_render.cu": ["-fmad=false"]}
 HEADERS = ["pg_math.cuh", "pg_model.h", "pg_tile.cuh", "pg_dynamics.cuh", "pg_collide.cuh", "pg_linalg.cuh", "pg_small.cuh", "pg_pgs.cuh", "pg_general.cuh", "pg_mlp.h",
-           "pg_newton.cuh", "pg_kernels.h"]
+           "pg_newton.cuh", "pg_kernels.h", "pg_lane.h", "pg_lane.cuh"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 

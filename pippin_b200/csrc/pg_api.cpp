@@ -16,6 +16,8 @@
 
 #include "../../include/pippin_b200.h"
 #include "pg_kernels.h"
+#include "pg_lane.h"
+#include "pg_math.cuh"
 #include "pg_mlp.h"
 #include "pg_model.h"
 
@@ -406,6 +408,14 @@ struct Handle {
   LearnArgs learn{};
   bool mlp_loaded = false;
   std::vector<double> base_params;
+  // the one- and four-lane substeps: whether the model takes one (STEP_*),
+  // whether the caller asked for a phase-kernel shape instead, and their copy
+  // of the parameter blocks ([32 envs][k][lane], made by the first
+  // pg_set_param that changes a physical parameter; until then every env
+  // reads env 0's block)
+  int kind = STEP_PHASES;
+  bool forced_shape = false;
+  double* prm_lanes = nullptr;
   int warm_mode = WARM_REF_PREV_QACC;
   SubstepCfg cfg{{16, 4, 0}, {32, 4, 0}, {16, 4, 0}};
   int sm_count = 0;
@@ -485,7 +495,7 @@ StepArgs make_args(Handle* h) {
 
 // Workspace layouts of the smooth-dynamics phase (w) and the Newton phase
 // (wn), the Newton phase's tile scratch (s) and the per-env work record (k).
-void layouts(const HostModel& m, int maxcon, int maxrows, WsLayout* w, WsLayout* wn, ScrLayout* s, WorkLayout* k) {
+void layouts(const HostModel& m, int maxcon, int maxrows, bool lane, WsLayout* w, WsLayout* wn, ScrLayout* s, WorkLayout* k) {
   int off = 0;
   auto take = [&](int n) {
     int o = off;
@@ -587,7 +597,7 @@ void layouts(const HostModel& m, int maxcon, int maxrows, WsLayout* w, WsLayout*
   k->rinvh = take(nv);
   k->meta = take(K_META_SIZE);
   k->geoms = take(ng * G_STRIDE);
-  k->contacts = take(maxcon * C_STRIDE);
+  k->contacts = take(maxcon * (lane ? std::max<int>(C_STRIDE, LC_STRIDE) : C_STRIDE));
   k->stride = off;
 
   off = 0;
@@ -615,7 +625,7 @@ std::vector<int> dmodel_pointer_fields() {
 #define PF(f) o.push_back((int)offsetof(DModel, f))
   PF(body_parent); PF(body_jntadr); PF(body_jntnum); PF(body_dofadr); PF(body_dofnum); PF(body_lastdof);
   PF(body_dofmask); PF(body_pos); PF(body_quat); PF(level_adr); PF(level_body); PF(child_adr); PF(child_list);
-  PF(jnt_type); PF(jnt_qposadr); PF(jnt_dofadr); PF(jnt_limited); PF(jnt_pos); PF(jnt_axis); PF(jnt_range);
+  PF(jnt_type); PF(jnt_qposadr); PF(jnt_dofadr); PF(jnt_limited); PF(jnt_pos); PF(jnt_axis); PF(jnt_unit); PF(jnt_range);
   PF(jnt_stiffness); PF(jnt_springref); PF(dof_body); PF(dof_parent); PF(dof_armature); PF(dof_block);
   PF(block_adr); PF(dofact_adr); PF(dofact_u); PF(dofact_coef); PF(geom_type); PF(geom_body); PF(geom_dataid);
   PF(geom_pos); PF(geom_quat); PF(pair_g); PF(cam_body); PF(cam_pos); PF(cam_quat); PF(act_gear);
@@ -624,6 +634,7 @@ std::vector<int> dmodel_pointer_fields() {
   PF(eq_solimp); PF(qpos0); PF(hull_vadr); PF(hull_vnum); PF(hull_vert); PF(hull_fadr); PF(hull_fnum);
   PF(hull_face); PF(hull_fvadr); PF(hull_fvnum); PF(hull_fv); PF(hull_eadr); PF(hull_enum); PF(hull_edge);
   PF(hull_eface); PF(hull_nbadr); PF(hull_nbnum); PF(hull_nb); PF(hull_seed);
+  PF(trunk); PF(limb_adr); PF(limb_body); PF(body_gadr); PF(pair_pack); PF(dof_limq); PF(dof_range);
 #undef PF
   return o;
 }
@@ -714,12 +725,59 @@ int set_const_range(Handle* h, int64_t start, int64_t end) {
   return launch_status(launch_set_const(a, fit(h->cfg.smooth, end - start), nullptr, (int)(end - start), h->stream));
 }
 
+// Whether the handle's substeps run on one or four lanes an env. Measured
+// against the three phase kernels (us a substep, single-substep calls, 4 / 512
+// / 4096 / 16384 envs):
+//   one lane, models without constraint rows: pendulum 11 / 13 / 13 / 13
+//   against 45 / 45 / 52 / 118, cartpole 17 / 20 / 21 / 21 against 56 / 54 /
+//   63 / 163. With rows a lane's Newton loses to the phase kernels in the
+//   middle of the range (a 6-hinge chain: 62 / 145 / 200 / 259 against 94 /
+//   130 / 167 / 446), so such models go elsewhere;
+//   four lanes, one tree with rows possible: Ant 65 / 95 / 113 / 217 against
+//   103 / 129 / 166 / 541, three limbs of 12 dofs 65 / 129 / 168 / 311 against
+//   110 / 161 / 257 / 653, five limbs of 16 dofs 78 / 181 / 244 / 509 against
+//   113 / 193 / 288 / 929, the 6-hinge chain 55 / 106 / 126 / 249 against the
+//   94 / 130 / 167 / 446 above.
+// The choice is the model's, not the call's: a range steps to the bits of the
+// whole.
+bool use_lanes(const Handle* h) {
+  return h->kind != STEP_PHASES && !h->forced_shape && h->dm.solver == SOLVER_NEWTON && h->warm_mode != WARM_LEARNED;
+}
+LaneArgs lane_args(const Handle* h, int64_t count) {
+  LaneArgs p{};
+  p.prm = h->prm_lanes ? h->prm_lanes : h->params;
+  p.uniform = h->prm_lanes ? 0 : 1;
+  p.sms = h->sm_count;
+  // a full warp's worth of envs only once every SM sub-partition has a warp:
+  // below that fewer envs a warp end the Newton loop sooner
+  const int most = h->kind == STEP_QUADS ? 8 : 32;
+  p.lanes = 1;
+  while (p.lanes < most && count > (int64_t)p.lanes * 4 * h->sm_count) p.lanes *= 2;
+  return p;
+}
+// nstep substeps of [start, end) one lane per env, LANE_CHUNK a launch
+constexpr int64_t LANE_CHUNK = 64;
+int enqueue_lanes(Handle* h, StepArgs a, int64_t start, int64_t end, int64_t nstep) {
+  a.start = (int)start;
+  a.count = (int)(end - start);
+  a.nstep = (int)nstep;
+  LaneArgs p = lane_args(h, end - start);
+  for (int64_t k = 0; k < nstep; k += LANE_CHUNK) {
+    p.sidx = (int)k;
+    p.nsub = (int)std::min(LANE_CHUNK, nstep - k);
+    cudaError_t e = h->kind == STEP_QUADS ? launch_quad(a, p, h->stream) : launch_lane(a, p, h->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "substep launch");
+  }
+  return PG_OK;
+}
+
 // One substep, or the graph-replayed sequence of `nstep` substeps, of envs
 // [start, end) on the handle's stream.
 int enqueue_substeps(Handle* h, StepArgs a, int64_t start, int64_t end, int64_t nstep) {
   a.start = (int)start;
   a.count = (int)(end - start);
   a.nstep = (int)nstep;
+  if (use_lanes(h)) return enqueue_lanes(h, a, start, end, nstep);
   SubstepCfg c = fit(h->cfg, end - start);
   for (int64_t k = 0; k < nstep; k++) {
     a.sidx = (int)k;
@@ -847,6 +905,43 @@ void read_param(const DModel& d, const double* prm, int p, int64_t id, double* o
   }
 }
 
+// Whether a pair of geoms can touch under the model's own masks.
+bool pair_masked(const HostModel& m, size_t p) {
+  int a = m.pairs[2 * p], b = m.pairs[2 * p + 1];
+  return !(m.geom_contype[a] & m.geom_conaffinity[b]) && !(m.geom_contype[b] & m.geom_conaffinity[a]);
+}
+// The substep a model's Newton steps take (STEP_*): see the rule's figures at
+// the definition of use_lanes. Both kernels hold one tree of at most 16 dofs
+// and need the bodies depth first and explicit damping.
+int step_kind(const HostModel& m, const DModel& d) {
+  if (m.nv < 1 || m.nv > LANE_NV || m.nq > LANE_NQ || m.dof_blocks.size() != 2 || m.neq > 0 || m.integrator != 0)
+    return STEP_PHASES;
+  std::vector<int> path = {0};
+  for (int b = 1; b < m.nbody; b++) {
+    while (!path.empty() && path.back() != m.body_parent[b]) path.pop_back();
+    if (path.empty() || (int)path.size() > LANE_DEPTH) return STEP_PHASES;
+    path.push_back(b);
+  }
+  bool rows = false;
+  for (int j = 0; j < m.njnt; j++) rows |= m.jnt_limited[j] && (m.jnt_type[j] == JNT_HINGE || m.jnt_type[j] == JNT_SLIDE);
+  for (size_t p = 0; 2 * p + 1 < m.pairs.size(); p++) rows |= !pair_masked(m, p);
+  if (!rows && d.limb_n < 3) return STEP_LANES;
+  // four lanes: limbs that are chains, primitive pairs, at most one violated
+  // side a limit, geoms in body order
+  if (d.limb_n < 0 || d.trunk_n > LANE_DEPTH || d.limb_max > LANE_DEPTH || m.nu > QUAD_NU || m.ngeom > LANE_GEOM)
+    return STEP_PHASES;
+  for (int g = 1; g < m.ngeom; g++)
+    if (m.geom_body[g] < m.geom_body[g - 1]) return STEP_PHASES;
+  for (size_t p = 0; p + 1 < m.pairs.size(); p += 2) {
+    int a = m.geom_type[m.pairs[p]], b = m.geom_type[m.pairs[p + 1]];
+    if (a == GEOM_MESH || b == GEOM_MESH) return STEP_PHASES;
+    if ((a == GEOM_CYLINDER && b != GEOM_PLANE) || (b == GEOM_CYLINDER && a != GEOM_PLANE)) return STEP_PHASES;
+  }
+  for (int j = 0; j < m.njnt; j++)
+    if (m.jnt_limited[j] && !(m.jnt_range[2 * j] <= m.jnt_range[2 * j + 1])) return STEP_PHASES;
+  return STEP_QUADS;
+}
+
 int build_device_model(Handle* h) {
   HostModel& m = h->hm;
   DModel& d = h->dm;
@@ -897,6 +992,38 @@ int build_device_model(Handle* h) {
     }
   }
   dofact_adr[nv] = (int)dofact_u.size();
+  // trunk and limbs: the quad substep walks the limbs side by side
+  std::vector<int> trunk, limb_adr = {0}, limb_body, body_gadr(nb + 1, 0);
+  auto nchild = [&](int b) { return child_adr[b + 1] - child_adr[b]; };
+  int end = 0;
+  while (nchild(end) == 1) {
+    end = child_list[child_adr[end]];
+    trunk.push_back(end);
+  }
+  bool chains = true;
+  for (int c = child_adr[end + 1] - 1; c >= child_adr[end]; c--) {
+    int b = child_list[c];
+    for (;; b = child_list[child_adr[b]]) {
+      limb_body.push_back(b);
+      if (nchild(b) != 1) break;
+    }
+    chains = chains && nchild(b) == 0;
+    limb_adr.push_back((int)limb_body.size());
+  }
+  d.trunk_n = (int)trunk.size();
+  d.limb_n = chains ? (int)limb_adr.size() - 1 : -1;
+  d.limb_max = 0;
+  for (int l = 0; l < d.limb_n; l++) d.limb_max = std::max(d.limb_max, limb_adr[l + 1] - limb_adr[l]);
+  for (int b = 0; b <= nb; b++)
+    while (body_gadr[b] < m.ngeom && m.geom_body[body_gadr[b]] < b) body_gadr[b]++;
+  std::vector<int> dof_limq(std::max(nv, 1), -1);
+  std::vector<double> dof_range(2 * std::max(nv, 1), 0.0);
+  for (int j = 0; j < m.njnt; j++)
+    if (m.jnt_limited[j] && (m.jnt_type[j] == JNT_HINGE || m.jnt_type[j] == JNT_SLIDE)) {
+      dof_limq[m.jnt_dofadr[j]] = m.jnt_qposadr[j];
+      dof_range[2 * m.jnt_dofadr[j]] = m.jnt_range[2 * j];
+      dof_range[2 * m.jnt_dofadr[j] + 1] = m.jnt_range[2 * j + 1];
+    }
   // work caps: every candidate pair at its largest manifold
   int maxcon = 0;
   for (size_t k = 0; k + 1 < m.pairs.size(); k += 2) maxcon += max_hits(m.geom_type[m.pairs[k]], m.geom_type[m.pairs[k + 1]]);
@@ -1053,12 +1180,24 @@ int build_device_model(Handle* h) {
   ADDI(jnt_limited, m.jnt_limited);
   ADDD(jnt_pos, m.jnt_pos);
   ADDD(jnt_axis, m.jnt_axis);
+  std::vector<double> jnt_unit(m.jnt_axis);
+  for (int j = 0; j < m.njnt; j++) {
+    V3 u = normalized(ld3(&jnt_unit[3 * j]));
+    st3(&jnt_unit[3 * j], u);
+  }
+  ADDD(jnt_unit, jnt_unit);
   ADDD(jnt_range, m.jnt_range);
   ADDD(jnt_stiffness, m.jnt_stiffness);
   ADDD(jnt_springref, m.jnt_springref);
   ADDI(dof_body, m.dof_body);
   ADDI(dof_parent, m.dof_parent);
   ADDD(dof_armature, m.dof_armature);
+  ADDI(dof_limq, dof_limq);
+  ADDD(dof_range, dof_range);
+  ADDI(trunk, trunk);
+  ADDI(limb_adr, limb_adr);
+  ADDI(limb_body, limb_body);
+  ADDI(body_gadr, body_gadr);
   ADDI(dof_block, dof_block);
   ADDI(block_adr, m.dof_blocks);
   ADDI(dofact_adr, dofact_adr);
@@ -1070,6 +1209,12 @@ int build_device_model(Handle* h) {
   ADDD(geom_pos, m.geom_pos);
   ADDD(geom_quat, m.geom_quat);
   ADDI(pair_g, m.pairs);
+  std::vector<int> pair_pack(m.pairs.size() / 2);
+  for (size_t p = 0; p < pair_pack.size(); p++) {
+    int g1 = m.pairs[2 * p], g2 = m.pairs[2 * p + 1];
+    pair_pack[p] = (g1 & 255) | (g2 & 255) << 8 | m.geom_type[g1] << 16 | m.geom_type[g2] << 20;
+  }
+  ADDI(pair_pack, pair_pack);
   ADDI(cam_body, m.cam_body);
   ADDD(cam_pos, m.cam_pos);
   ADDD(cam_quat, m.cam_quat);
@@ -1157,7 +1302,8 @@ int build_device_model(Handle* h) {
     for (int k = 0; k < 3; k++) bp[d.p_bias + 3 * u + k] = m.act_bias[3 * u + k];
   }
   for (int k = 0; k < m.nq; k++) bp[d.p_qpos_reset + k] = m.qpos_reset[k];
-  layouts(m, maxcon, maxrows, &h->w, &h->wn, &h->s, &h->k);
+  h->kind = step_kind(m, d);
+  layouts(m, maxcon, maxrows, h->kind == STEP_QUADS, &h->w, &h->wn, &h->s, &h->k);
   return PG_OK;
 }
 
@@ -1166,7 +1312,7 @@ void destroy(pg_handle* h) {
   cudaSetDevice(h->device);
   clear_graphs(h);
   void* ptrs[] = {h->d_model, h->qpos, h->qvel, h->ctrl, h->qacc, h->applied, h->params, h->iters, h->ncon,
-                  h->nrows, h->status, h->scratch, h->work, h->prev_con, h->prev_ncon, h->queue, h->order, h->b_ctrl.p, h->b_qout.p, h->b_poses_g.p,
+                  h->nrows, h->status, h->scratch, h->prm_lanes, h->work, h->prev_con, h->prev_ncon, h->queue, h->order, h->b_ctrl.p, h->b_qout.p, h->b_poses_g.p,
                   h->b_poses_c.p, h->b_dbg.p, h->b_vals.p, h->b_ids.p, h->learn.items, h->learn.feat, h->learn.force,
                   h->learn.rows, (void*)h->learn.mlp_w, (void*)h->learn.mlp_f, (void*)h->learn.mlp_err};
   for (void* p : ptrs)
@@ -1209,6 +1355,12 @@ int internal_step_args(pg_handle* h, int64_t start, int64_t end, int64_t nstep, 
   *stream = h->stream;
   *device = h->device;
   return PG_OK;
+}
+// The same step one lane per env, where the handle's substeps run so.
+bool internal_step_lanes(pg_handle* h, const StepArgs& a, int64_t start, int64_t end, int64_t nstep, int* rc) {
+  if (!use_lanes(h)) return false;
+  *rc = enqueue_lanes(h, a, start, end, nstep);
+  return true;
 }
 void internal_set_error(const std::string& msg) { g_err = msg; }
 }  // namespace pg
@@ -1323,6 +1475,7 @@ int pg_step(pg_handle* h, int64_t start, int64_t end, int64_t nstep) {
   if (nstep < 0 || nstep > (1 << 30)) return fail(PG_ERR_INVALID, "nstep out of range");
   if (end == start || nstep == 0) return PG_OK;
   CK(cudaSetDevice(h->device));
+  if (use_lanes(h)) return enqueue_lanes(h, make_args(h), start, end, nstep);
   if (h->graph_version != h->version) {
     clear_graphs(h);
     h->graph_version = h->version;
@@ -1538,11 +1691,42 @@ int pg_set_param(pg_handle* h, int param, int64_t id, int64_t start, int64_t end
   CK(cudaSetDevice(h->device));
   // the values go to the device, where each env's parameter block takes them
   if ((rc = grow(h, h->b_vals, sizeof(double) * len))) return rc;
+  const bool physical = param != PG_PARAM_GEOM_RGBA && param != PG_PARAM_QPOS0;
+  const bool first = h->kind != STEP_PHASES && physical && !h->prm_lanes;
+  std::unique_ptr<double, cudaError_t (*)(void*)> fresh(nullptr, [](void* p) { return cudaFree(p); });
+  if (first) {
+    double* p = nullptr;
+    CK(cudaMalloc(&p, sizeof(double) * ((h->n + 31) / 32 * 32) * h->dm.pstride));
+    fresh.reset(p);
+  }
   CK(cudaMemcpyAsync(h->b_vals.p, values, sizeof(double) * len, cudaMemcpyHostToDevice, h->stream));
   CK(launch_apply_param(h->dm, h->params + start * h->dm.pstride, end - start, param, id, (const double*)h->b_vals.p, w,
                         m.nq, h->stream));
   if (param == PG_PARAM_BODY_MASS || param == PG_PARAM_BODY_INERTIA || param == PG_PARAM_BODY_IPOS) {
     if ((rc = set_const_range(h, start, end))) return rc;
+  }
+  // masks may now let pairs touch: a model that took one lane for want of
+  // rows leaves it
+  if ((param == PG_PARAM_GEOM_CONTYPE || param == PG_PARAM_GEOM_CONAFFINITY) && h->kind == STEP_LANES) h->kind = STEP_PHASES;
+  if (h->kind != STEP_PHASES && physical) {
+    const DModel& d = h->dm;
+    auto mirror = [&](int64_t e0, int64_t e1, int off, int cnt) {
+      return launch_mirror(h->params, h->prm_lanes, d.pstride, e0, e1, off, cnt, h->stream);
+    };
+    if (first) {
+      CK(launch_mirror(h->params, fresh.get(), d.pstride, 0, h->n, 0, d.pstride, h->stream));
+      h->prm_lanes = fresh.release();
+    } else {
+      const int at[] = {d.p_friction + (int)id, d.p_size + 3 * (int)id, 0, d.p_contype + (int)id, d.p_conaff + (int)id,
+                        d.p_mass + (int)id, d.p_damping + (int)id, d.p_gain + (int)id, d.p_bias + 3 * (int)id,
+                        d.p_inertia + 9 * (int)id, d.p_ipos + 3 * (int)id};
+      CK(mirror(start, end, at[param], param == PG_PARAM_BODY_INERTIA ? 9 : w));
+      if (param == PG_PARAM_BODY_MASS) CK(mirror(start, end, d.p_inertia + 9 * (int)id, 9));
+      if (param == PG_PARAM_BODY_MASS || param == PG_PARAM_BODY_INERTIA || param == PG_PARAM_BODY_IPOS) {
+        CK(mirror(start, end, d.p_body_invw, 2 * m.nbody));
+        CK(mirror(start, end, d.p_dof_invw, m.nv));
+      }
+    }
   }
   CK(cudaStreamSynchronize(h->stream));
   return PG_OK;
@@ -1744,6 +1928,8 @@ int pg_set_launch(pg_handle* h, int lanes_per_env, int envs_per_block) {
     if (envs_per_block > 0) p->tiles_per_block = envs_per_block;
   }
   CK(cudaSetDevice(h->device));
+  // a caller that names a shape gets the phase kernels in it
+  if (lanes_per_env > 0 || envs_per_block > 0) h->forced_shape = true;
   return apply_cfg(h, c);
 }
 
@@ -1771,6 +1957,7 @@ int pg_autotune(pg_handle* h, int64_t nstep) {
   if (h->n == 0) return PG_OK;
   if (nstep < 1) nstep = 1;
   CK(cudaSetDevice(h->device));
+  if (use_lanes(h)) return PG_OK;  // the one-lane-per-env substep has no shape to search
   const HostModel& m = h->hm;
   size_t n = h->n;
   // save the state the trial steps will overwrite

@@ -501,7 +501,7 @@ __device__ inline V3 p_centroid(const Poly& p) {
 // the farthest from it, the farthest from their line, the most isolated),
 // each taken within GEN_TIE: the first minimum, the last maximum. A clipped
 // regular polygon (a cylinder cap) offers many exact ties.
-__device__ __noinline__ int reduce_to_four_tie(DP* pts, int n) {
+__device__ __noinline__ inline int reduce_to_four_tie(DP* pts, int n) {
   if (n <= 4) return n;
   DP keep[4];
   double mn = INFINITY;
@@ -545,7 +545,7 @@ __device__ inline int clip_poly_cap(const V3* in, int n, V3 pn, double off, V3* 
 // within the margin (up to four); (first geom to second). The clip runs in `area` (10 cap
 // doubles: two polygon buffers of cap vertices, then cap kept points) when
 // given, else in the lane's own buffers of GEN_CLIP_CAP.
-__device__ __noinline__ void clip_faces(const Poly& r, int rf, const Poly& s, V3 n, double margin, Hits& out,
+__device__ __noinline__ inline void clip_faces(const Poly& r, int rf, const Poly& s, V3 n, double margin, Hits& out,
                                         double* area, int cap) {
   V3 nref = p_fn(r, rf);
   double dref = p_fd(r, rf, nref);

@@ -1,0 +1,41 @@
+// Launcher of the one-lane-per-env substep (pg_lane.cu).
+#pragma once
+#include <cuda_runtime.h>
+
+#include "pg_kernels.h"
+
+namespace pg {
+
+// which substep a model's Newton steps take: the three phase kernels, one
+// lane an env (no constraint rows possible), or four
+enum { STEP_PHASES = 0, STEP_LANES = 1, STEP_QUADS = 2 };
+// limits of the models the lane and quad kernels take (sizes of its per-lane arrays)
+constexpr int LANE_NV = 16;     // dofs
+constexpr int LANE_NQ = 24;     // positions
+constexpr int LANE_GEOM = 32;   // geoms
+constexpr int QUAD_NU = 32;     // actuators (quad)
+constexpr int LANE_DEPTH = 8;   // tree levels below the world
+// a contact in the lane's slice of the work record (doubles): point, normal,
+// first tangent, friction, D (0: not touching), the constant part of its
+// residual, its dof masks, residual and its change along the search direction
+enum { LC_POS = 0, LC_N = 3, LC_T = 6, LC_MU = 9, LC_D = 10, LC_OFF = 11, LC_MASK = 14, LC_E = 15, LC_P = 18,
+       LC_STRIDE = 21 };
+
+struct LaneArgs {
+  const double* prm;   // parameter blocks: see below
+  int uniform;         // 1: every env reads the block at prm; 0: blocks of 32 envs, [k][32], from env 0
+  int lanes;           // envs a warp takes (1..32)
+  int sms;             // SMs of the GPU
+  int sidx, nsub;      // substeps [sidx, sidx + nsub) of the call
+};
+
+// Substeps [p.sidx, p.sidx + p.nsub) of envs [a.start, a.start + a.count), one launch.
+cudaError_t launch_lane(const StepArgs& a, const LaneArgs& p, cudaStream_t s);
+// The same with four lanes per env (a.m.limb_n >= 0; p.lanes at most 8).
+cudaError_t launch_quad(const StepArgs& a, const LaneArgs& p, cudaStream_t s);
+// rows [off, off + len) of the parameter blocks of envs [start, end) into the
+// lane kernel's layout
+cudaError_t launch_mirror(const double* params, double* lanes, int pstride, int64_t start, int64_t end, int off, int len,
+                          cudaStream_t s);
+
+}  // namespace pg

@@ -30,6 +30,7 @@ namespace pg {
 // fills the launch arguments of pg_step for [start, end) (pg_api.cpp)
 int internal_step_args(pg_handle* h, int64_t start, int64_t end, int64_t nstep, StepArgs* a, SubstepCfg* cfg,
                        cudaStream_t* stream, int* device);
+bool internal_step_lanes(pg_handle* h, const StepArgs& a, int64_t start, int64_t end, int64_t nstep, int* rc);
 void internal_set_error(const std::string& msg);
 }  // namespace pg
 
@@ -89,6 +90,8 @@ extern "C" int pg_step_static(pg_handle* h, int64_t start, int64_t end, int64_t 
   int rc = pg::internal_step_args(h, start, end, nstep, &a, &cfg, &stream, &device);
   if (rc != PG_OK) return rc;
   if (end == start || nstep == 0) return PG_OK;
+  // one lane per env needs no tile scratch at all
+  if (pg::internal_step_lanes(h, a, start, end, nstep, &rc)) return rc;
   unsigned char* base = nullptr;  // internal_step_args made the handle's device current
   if ((rc = scratch_address(&base)) != PG_OK) return rc;
   // only the Newton phase uses tile scratch: its grid is capped by the array

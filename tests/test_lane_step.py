@@ -1,0 +1,163 @@
+"""The substep with one lane or four lanes per env (pg_lane.cu, pg_quad.cu)
+against the oracle, step by step from the same states: models without rows
+(one lane; 4 and 8 dofs of register arrays), chains, two limbs, three and more
+on a trunk (four lanes; 8, 12, 14 and 16), a second round of limbs, a tree
+that neither takes, and batches around the sizes where warps and blocks fill.
+
+Tolerance: the per-step bar of the other parity tests, 1e-10 of the largest
+component (a step's rounding is below 1e-14 of it, the factorisations and the
+Newton exit leave four digits more).
+"""
+import numpy as np
+import pytest
+
+from oracle.oracle import CTRL, QACC, QPOS, QVEL, Oracle
+from pippin_b200 import CudaPhysics, Field, Param, WarmStart, mjcf, scenes
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-10
+
+OPT = '<compiler angle="degree"/><option timestep="0.004" tolerance="1e-10" iterations="30"/>'
+FLOOR = '<geom type="plane" size="5 5 .1" friction="0.8 0.1 0.1"/>'
+
+
+def _limb(k, geom, free_end=True):
+    """Two hinges, the first with a range, out along the k-th direction."""
+    a = 2.0 * np.pi * k / 5.0
+    x, y = 0.25 * np.cos(a), 0.25 * np.sin(a)
+    g = {"capsule": f'<geom type="capsule" fromto="0 0 0 {x:.4f} {y:.4f} -0.1" size="0.05"/>',
+         "sphere": f'<geom type="sphere" pos="{x:.4f} {y:.4f} -0.1" size="0.07"/>',
+         "box": f'<geom type="box" pos="{x:.4f} {y:.4f} -0.1" size="0.06 0.05 0.04" euler="10 20 30"/>'}[geom]
+    return (f'<body pos="{0.4 * x:.4f} {0.4 * y:.4f} 0" euler="0 0 {7 * k}">'
+            f'<joint name="a{k}" axis="0 0 1" range="-20 20" limited="true" damping="0.3" armature="0.02"/>{g}'
+            f'<body pos="{x:.4f} {y:.4f} -0.1"><joint name="b{k}" axis="{y:.4f} {-x:.4f} 0" pos="0.01 0 0.02" '
+            f'stiffness="3" armature="0.01"/>{g}</body></body>')
+
+
+def _star(limbs, root='<freejoint/>', geoms=("capsule", "sphere", "box"), extra=""):
+    body = "".join(_limb(k, geoms[k % len(geoms)]) for k in range(limbs))
+    motors = "".join(f'<motor joint="a{k}" gear="4"/><position joint="b{k}" kp="6" kv="0.3"/>' for k in range(limbs))
+    return (f'<mujoco>{OPT}<worldbody>{FLOOR}{extra}<body pos="0 0 0.35">{root}'
+            f'<geom type="sphere" size="0.1" density="400"/>{body}</body></worldbody><actuator>{motors}</actuator></mujoco>')
+
+
+def _chain(n, ball=False):
+    s, e = "", ""
+    for k in range(n):
+        ax = ["0 0 1", "0 1 0", "1 0 0"][k % 3]
+        j = '<joint type="ball" damping="0.05"/>' if ball and k == n - 1 else (
+            f'<joint name="j{k}" axis="{ax}" range="-40 40" limited="true" armature="0.02" damping="{0.1 * (k % 2)}"/>')
+        s += (f'<body pos="0.12 0 0" euler="0 {5 * (k % 2)} 0">{j}'
+              '<geom type="capsule" fromto="0 0 0 0.12 0 0" size="0.035"/>')
+        e += "</body>"
+    return (f'<mujoco>{OPT}<worldbody>{FLOOR}<body pos="0 0 0.1"><geom type="box" size="0.03 0.03 0.03"/>{s}{e}</body>'
+            '</worldbody><actuator><motor joint="j0" gear="3"/></actuator></mujoco>')
+
+
+MODELS = {
+    "pendulum": scenes.pendulum_xml(),                     # one lane, 4
+    "chain_7_ball": _chain(5, ball=True),                  # four lanes, 8: a trunk alone, a ball
+    "chain_6": _chain(6),                                  # four lanes, 8: as deep as it goes
+    "two_limbs": _star(2),                                 # four lanes, 12
+    "arm3d": scenes.arm3d_xml(),                           # one lane, 8: ball, slide, offsets
+    "hinge_3_limbs": _star(3, root='<joint axis="0 0 1" damping="0.2" armature="0.05"/>'),   # four lanes, 8
+    "free_3_limbs": _star(3),                              # four lanes, 12
+    "ant": scenes.ant_xml(timestep=0.004, tolerance=1e-10),                                 # four lanes, 14
+    "free_5_limbs": _star(5),                              # four lanes, 16: two rounds of limbs
+    # the phase kernels: a branching tree and a static body beside it
+    "static_box": _star(4, geoms=("capsule",), extra='<body pos="0.3 0 0"><geom type="box" size="0.1 0.5 0.05"/></body>'),
+}
+
+
+def _states(m, n, rng):
+    q = np.tile(np.array(m.qpos0), (n, 1))
+    for j in range(m.njnt):
+        a, t = m.jnt_qposadr[j], m.jnt_type[j]
+        if t == mjcf.JNT_FREE:
+            q[:, a:a + 2] = rng.uniform(-0.2, 0.2, (n, 2))
+            q[:, a + 2] = rng.uniform(0.1, 0.5, n)
+            a += 3
+        if t in (mjcf.JNT_FREE, mjcf.JNT_BALL):
+            w = rng.normal(0, 1, (n, 4)) * 0.15 + np.array([1.0, 0, 0, 0])
+            q[:, a:a + 4] = w / np.linalg.norm(w, axis=1, keepdims=True)
+        elif t == mjcf.JNT_HINGE:
+            q[:, a] += rng.uniform(-0.8, 0.8, n)
+        else:
+            q[:, a] += rng.uniform(-0.1, 0.1, n)
+    return q, rng.normal(0, 1.0, (n, m.nv))
+
+
+def _rel(a, b):
+    return float(np.max(np.abs(a - b)) / max(float(np.max(np.abs(b))), 1.0))
+
+
+@pytest.mark.parametrize("name", list(MODELS))
+@pytest.mark.parametrize("n", [1, 8, 33, 700])
+def test_step_matches_oracle(name, n):
+    m = mjcf.load_string(MODELS[name])
+    blob = mjcf.to_blob(m)
+    g, o = CudaPhysics(blob, n), Oracle(blob, n, threads=8)
+    o.set_solver(tolerance=1e-10, iterations=30)
+    g.set_solver(tolerance=1e-10, iterations=30, warm=int(WarmStart.REF_PREV_QACC))
+    rng = np.random.default_rng(n)
+    q, v = _states(m, n, rng)
+    g.set(Field.QPOS, range(n), q)
+    g.set(Field.QVEL, range(n), v)
+    rows = 0
+    for t in range(6):
+        if t == 3:  # per-env parameters: the kernels' own copy of them
+            mass = np.asarray(m.body_mass[m.nbody - 1]) * rng.uniform(0.7, 1.5, (n, 1))
+            fric = rng.uniform(0.4, 1.1, (n, 1))
+            for pid, elem, val in ((5, m.nbody - 1, mass), (0, 0, fric), (6, m.nv - 1, fric)):
+                g.set_param(Param(pid), elem, range(n), val)
+                o.set_param(pid, elem, val, 0, n)
+        if m.nu:
+            g.set(Field.CTRL, range(n), rng.uniform(-1, 1, (n, m.nu)))
+        for fg, fo in ((Field.QPOS, QPOS), (Field.QVEL, QVEL), (Field.QACC, QACC), (Field.CTRL, CTRL)):
+            if g.dims().width(fg):
+                o.set(fo, g.get(fg, range(n)))
+        g.step(range(n), 1)
+        o.step(0, n, 1)
+        for fg, fo in ((Field.QACC, QACC), (Field.QVEL, QVEL), (Field.QPOS, QPOS)):
+            assert _rel(g.get(fg, range(n)), o.get(fo)) < TOL, (t, fg)
+        sg, so = g.stats(), o.stats()
+        np.testing.assert_array_equal(sg["ncon"], so["ncon"])
+        np.testing.assert_array_equal(sg["nrows"], so["nrows"])
+        assert not sg["status"].any()
+        rows += int(sg["nrows"].sum())
+    assert rows > 0 or n < 33 or name in ("pendulum", "arm3d")  # (these two have no contacts and no limits)
+
+
+def test_named_shape_runs_the_phase_kernels():
+    """set_launch names a shape of the phase kernels: the step then takes
+    them, and agrees with the default within the step tolerance."""
+    n = 100
+    m = mjcf.load_string(MODELS["ant"])
+    blob = mjcf.to_blob(m)
+    a, b = CudaPhysics(blob, n), CudaPhysics(blob, n)
+    b.set_launch(16, 4)
+    q, v = _states(m, n, np.random.default_rng(3))
+    for p in (a, b):
+        p.set(Field.QPOS, range(n), q)
+        p.set(Field.QVEL, range(n), v)
+        p.step(range(n), 2)
+    assert _rel(a.get(Field.QACC, range(n)), b.get(Field.QACC, range(n))) < TOL
+
+
+def test_long_calls_and_cold_start():
+    """A call longer than one launch takes, and the cold start, from one state
+    give the bits of single steps."""
+    n, t = 40, 130
+    m = mjcf.load_string(MODELS["free_5_limbs"])
+    blob = mjcf.to_blob(m)
+    a, b = CudaPhysics(blob, n), CudaPhysics(blob, n)
+    q, v = _states(m, n, np.random.default_rng(9))
+    for p in (a, b):
+        p.set_solver(warm=int(WarmStart.COLD))
+        p.set(Field.QPOS, range(n), q)
+        p.set(Field.QVEL, range(n), v)
+    a.step(range(n), t)
+    for _ in range(t):
+        b.step(range(n), 1)
+    for f in (Field.QPOS, Field.QVEL, Field.QACC):
+        np.testing.assert_array_equal(a.get(f, range(n)), b.get(f, range(n)))

@@ -888,20 +888,24 @@ bool validate_param(const HostModel& m, int p, int64_t id, const double* v, std:
 }
 
 
-void read_param(const DModel& d, const double* prm, int p, int64_t id, double* o, int nq) {
+// Where a parameter's values sit in a parameter block: the first one's place
+// and the distance between them.
+int param_offset(const DModel& d, int p, int64_t id, int* step) {
+  const int i = (int)id;
+  *step = p == PG_PARAM_BODY_INERTIA ? 4 : 1;  // the diagonal of a 3 x 3
   switch (p) {
-    case PG_PARAM_GEOM_FRICTION: o[0] = prm[d.p_friction + id]; break;
-    case PG_PARAM_GEOM_SIZE: for (int k = 0; k < 3; k++) o[k] = prm[d.p_size + 3 * id + k]; break;
-    case PG_PARAM_GEOM_RGBA: for (int k = 0; k < 4; k++) o[k] = prm[d.p_rgba + 4 * id + k]; break;
-    case PG_PARAM_GEOM_CONTYPE: o[0] = prm[d.p_contype + id]; break;
-    case PG_PARAM_GEOM_CONAFFINITY: o[0] = prm[d.p_conaff + id]; break;
-    case PG_PARAM_BODY_MASS: o[0] = prm[d.p_mass + id]; break;
-    case PG_PARAM_DOF_DAMPING: o[0] = prm[d.p_damping + id]; break;
-    case PG_PARAM_ACTUATOR_GAIN: o[0] = prm[d.p_gain + id]; break;
-    case PG_PARAM_ACTUATOR_BIAS: for (int k = 0; k < 3; k++) o[k] = prm[d.p_bias + 3 * id + k]; break;
-    case PG_PARAM_BODY_INERTIA: for (int k = 0; k < 3; k++) o[k] = prm[d.p_inertia + 9 * id + 4 * k]; break;
-    case PG_PARAM_BODY_IPOS: for (int k = 0; k < 3; k++) o[k] = prm[d.p_ipos + 3 * id + k]; break;
-    case PG_PARAM_QPOS0: for (int k = 0; k < nq; k++) o[k] = prm[d.p_qpos_reset + k]; break;
+    case PG_PARAM_GEOM_FRICTION: return d.p_friction + i;
+    case PG_PARAM_GEOM_SIZE: return d.p_size + 3 * i;
+    case PG_PARAM_GEOM_RGBA: return d.p_rgba + 4 * i;
+    case PG_PARAM_GEOM_CONTYPE: return d.p_contype + i;
+    case PG_PARAM_GEOM_CONAFFINITY: return d.p_conaff + i;
+    case PG_PARAM_BODY_MASS: return d.p_mass + i;
+    case PG_PARAM_DOF_DAMPING: return d.p_damping + i;
+    case PG_PARAM_ACTUATOR_GAIN: return d.p_gain + i;
+    case PG_PARAM_ACTUATOR_BIAS: return d.p_bias + 3 * i;
+    case PG_PARAM_BODY_INERTIA: return d.p_inertia + 9 * i;
+    case PG_PARAM_BODY_IPOS: return d.p_ipos + 3 * i;
+    default: return d.p_qpos_reset;
   }
 }
 
@@ -1717,10 +1721,9 @@ int pg_set_param(pg_handle* h, int param, int64_t id, int64_t start, int64_t end
       CK(launch_mirror(h->params, fresh.get(), d.pstride, 0, h->n, 0, d.pstride, h->stream));
       h->prm_lanes = fresh.release();
     } else {
-      const int at[] = {d.p_friction + (int)id, d.p_size + 3 * (int)id, 0, d.p_contype + (int)id, d.p_conaff + (int)id,
-                        d.p_mass + (int)id, d.p_damping + (int)id, d.p_gain + (int)id, d.p_bias + 3 * (int)id,
-                        d.p_inertia + 9 * (int)id, d.p_ipos + 3 * (int)id};
-      CK(mirror(start, end, at[param], param == PG_PARAM_BODY_INERTIA ? 9 : w));
+      int step;
+      const int off = param_offset(d, param, id, &step);
+      CK(mirror(start, end, off, param == PG_PARAM_BODY_INERTIA ? 9 : w));
       if (param == PG_PARAM_BODY_MASS) CK(mirror(start, end, d.p_inertia + 9 * (int)id, 9));
       if (param == PG_PARAM_BODY_MASS || param == PG_PARAM_BODY_INERTIA || param == PG_PARAM_BODY_IPOS) {
         CK(mirror(start, end, d.p_body_invw, 2 * m.nbody));
@@ -1746,10 +1749,13 @@ int pg_get_param(pg_handle* h, int param, int64_t id, int64_t start, int64_t end
     return fail(PG_ERR_INVALID, std::string(param_name(param)) + ": id " + std::to_string(id) + " out of range");
   if (end == start) return PG_OK;
   CK(cudaSetDevice(h->device));
-  std::vector<double> blk;
-  if ((rc = read_params(h, start, end, blk))) return rc;
-  for (int64_t k = 0; k < end - start; k++) read_param(h->dm, blk.data() + k * h->dm.pstride, param, id, out + k * w, m.nq);
-  return PG_OK;
+  // gathered on the device: the whole blocks (3.4 KB an Ant env) took 3.5 ms
+  // to bring back for 8192 envs, one parameter's values a few microseconds
+  if ((rc = grow(h, h->b_vals, sizeof(double) * len))) return rc;
+  int step = 1, off = param_offset(h->dm, param, id, &step);
+  CK(launch_read_param(h->params + start * h->dm.pstride, h->dm.pstride, end - start, off, w, step, (double*)h->b_vals.p,
+                       h->stream));
+  return copy_rows_d2h(h, out, (const double*)h->b_vals.p, 0, end - start, w);
 }
 
 int pg_appearance(pg_handle* h, int64_t start, int64_t end, pg_geom_appearance* out, size_t len) {

@@ -730,6 +730,18 @@ cudaError_t launch_apply_param(const DModel& d, double* params, int64_t count, i
   return cudaGetLastError();
 }
 
+__global__ void read_param_kernel(const double* params, int pstride, int64_t count, int off, int w, int step, double* out) {
+  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < count * w) out[i] = params[i / w * pstride + off + (int)(i % w) * step];
+}
+
+cudaError_t launch_read_param(const double* params, int pstride, int64_t count, int off, int w, int step, double* out,
+                              cudaStream_t s) {
+  if (count <= 0 || w <= 0) return cudaSuccess;
+  read_param_kernel<<<(unsigned)((count * w + 127) / 128), 128, 0, s>>>(params, pstride, count, off, w, step, out);
+  return cudaGetLastError();
+}
+
 __global__ void hull_support_kernel(const __grid_constant__ DModel m, int mesh, const double* dirs, int n,
                                     int* vertex) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -42,6 +42,9 @@ cudaError_t launch_reset(const StepArgs& a, const int64_t* ids, int n, cudaStrea
 // params[e * pstride ..] takes values v[e][w] of parameter p, element id, for e < count
 cudaError_t launch_apply_param(const DModel& d, double* params, int64_t count, int p, int64_t id, const double* v, int w,
                                int nq, cudaStream_t s);
+// out[e][k] = params[e * pstride + off + k * step] for e < count, k < w
+cudaError_t launch_read_param(const double* params, int pstride, int64_t count, int off, int w, int step, double* out,
+                              cudaStream_t s);
 // vertex[i] = the hull support walk of mesh `mesh` along dirs[i] (mesh frame; device memory)
 cudaError_t launch_hull_support(const DModel& m, int mesh, const double* dirs, int n, int* vertex, cudaStream_t s);
 

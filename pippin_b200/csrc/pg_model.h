@@ -199,7 +199,6 @@ __host__ __device__ inline void apply_param(const DModel& d, double* prm, int p,
   }
 }
 
-
 // Per-tile shared-memory workspace (offsets in doubles). The `tree` region
 // (poses, inertias, velocities, forces) is dead once the contacts are built
 // and is reused by the factorisations and Newton (`fac` .. `warm`).
@@ -283,7 +282,8 @@ struct EnvState {
 // impulses (normal, tangent 1, tangent 2)
 enum { P_POS = 0, P_T1 = 3, P_T2 = 6, P_G1 = 9, P_G2 = 10, P_LAMBDA = 11, P_STRIDE = 14 };
 // PGS row record in tile scratch (doubles; solver.rs:18-36)
-enum { PR_KIND = 0, PR_SEP = 1, PR_MU = 2, PR_NORMAL = 3, PR_CONTACT = 4, PR_INVA = 5, PR_LAMBDA = 6, PR_STRIDE = 8 };
+enum { PR_KIND = 0, PR_SEP = 1, PR_MU = 2, PR_NORMAL = 3, PR_CONTACT = 4, PR_INVA = 5, PR_LAMBDA = 6, PR_SPAN = 7,
+       PR_STRIDE = 8 };
 enum { PK_NORMAL = 0, PK_FRICTION = 1, PK_BILATERAL = 2 };
 
 constexpr int MAX_PTR_FIELDS = 80;

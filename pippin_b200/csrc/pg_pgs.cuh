@@ -3,13 +3,18 @@
 //
 // Rows follow the reference's order: [normal, tangent 1, tangent 2] per
 // contact (every contact of the narrow phase, not only touching ones), then
-// the joint-limit sides within reach, then the joint equalities. The rows of
-// M^-1 J' are formed one per lane with the reference's solve (division by the
-// pivot, dot-product order of math.rs), so each lane's row matches the CPU
-// bit for bit up to FMA contraction. The sweeps are sequential over rows, as
-// Gauss-Seidel must be: every lane forms J_r . v itself in the reference's
-// summation order (no reduction tree), and the velocity update v += dl M^-1
-// J_r' runs one dof per lane. Impulses live in the row records.
+// the joint-limit sides within reach, then the joint equalities. A row touches
+// the dofs of one or two trees: only those entries of J and M^-1 J' are formed
+// and read (PR_SPAN), the others are zero.
+//
+// Gauss-Seidel is sequential over rows, but rows of separate islands (trees
+// joined by rows) share no velocity, so each lane sweeps islands of its own, in
+// row order, and the tile meets once a sweep for the largest change: the
+// sequential sweep's result to the bit (a sum's terms that are left out are
+// zero). Impulses live in the row records. With the whole tile on one row at a
+// time (48 dofs a product, two tile syncs a row) 1001 envs of 8 hulls took
+// 6.67 ms in this phase, now 1.43 ms; what bounds it now is the
+// latency of the row's loads, which are prefetched a row ahead.
 #pragma once
 #include "pg_newton.cuh"
 
@@ -18,6 +23,41 @@ namespace pg {
 constexpr double PGS_MAX_BIAS_VELOCITY = 1.0;  // solver.rs:34
 constexpr double PGS_TOLERANCE = 1e-5;         // solver.rs:36
 constexpr double PGS_MATCH_DIST2 = 0.01 * 0.01;  // solver.rs:255
+
+// The dof ranges [a0, a1) and [b0, b1) a row touches (one tree, or two in
+// ascending order), packed in its record's PR_SPAN.
+struct Span {
+  int a0, a1, b0, b1;
+  __device__ static Span of(double v) {
+    unsigned u = (unsigned)v;
+    return Span{(int)(u & 127), (int)(u >> 7 & 127), (int)(u >> 14 & 127), (int)(u >> 21 & 127)};
+  }
+};
+// the tree of a body's dofs, or -1
+__device__ inline int body_tree(const DModel& m, int b) {
+  unsigned long long mk = m.body_dofmask[b];
+  return mk ? m.dof_block[__ffsll((long long)mk) - 1] : -1;
+}
+// of trees t1 and t2 (-1: none)
+__device__ inline double pack_span(const DModel& m, int t1, int t2) {
+  if (t1 == t2) t2 = -1;
+  if (t1 < 0 || (t2 >= 0 && t2 < t1)) {
+    int t = t1;
+    t1 = t2;
+    t2 = t;
+  }
+  unsigned u = 0;
+  if (t1 >= 0) u |= (unsigned)m.block_adr[2 * t1] | (unsigned)m.block_adr[2 * t1 + 1] << 7;
+  if (t2 >= 0) u |= (unsigned)m.block_adr[2 * t2] << 14 | (unsigned)m.block_adr[2 * t2 + 1] << 21;
+  return (double)u;
+}
+// f(k) for the span's dofs in ascending order
+__device__ __forceinline__ void prefetch_row(const double* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+template <class F>
+__device__ __forceinline__ void span_each(const Span& s, F f) {
+  for (int k = s.a0; k < s.a1; k++) f(k);
+  for (int k = s.b0; k < s.b1; k++) f(k);
+}
 
 // Rows of the PGS problem (solver.rs:63-163) into J (stride nv) and R
 // (PR_* records). Returns the row count, capped at maxrows.
@@ -40,6 +80,7 @@ __device__ int pgs_rows(const Tile<G>& T, const DModel& m, const WsLayout& w, co
     const double* r = con + C_STRIDE * c;
     int g1 = (int)r[C_G1], g2 = (int)r[C_G2];
     double mu = fmax(prm[m.p_friction + g1], prm[m.p_friction + g2]);
+    double span = pack_span(m, body_tree(m, m.geom_body[g1]), body_tree(m, m.geom_body[g2]));
     for (int q = 0; q < 3; q++) {
       double* rr = R + PR_STRIDE * (3 * c + q);
       rr[PR_KIND] = q == 0 ? PK_NORMAL : PK_FRICTION;
@@ -49,10 +90,15 @@ __device__ int pgs_rows(const Tile<G>& T, const DModel& m, const WsLayout& w, co
       rr[PR_CONTACT] = c;
       rr[PR_INVA] = 0.0;
       rr[PR_LAMBDA] = 0.0;
+      rr[PR_SPAN] = span;
     }
   }
-  for (int it = lane; it < nc * nv; it += G) {
-    int c = it / nv, k = it % nv;
+  T.sync();
+  for (int it = lane; it < nc * 2 * m.maxbs; it += G) {
+    int c = it / (2 * m.maxbs), o = it % (2 * m.maxbs);
+    Span sp = Span::of(R[PR_STRIDE * 3 * c + PR_SPAN]);
+    int k = o < m.maxbs ? sp.a0 + o : sp.b0 + o - m.maxbs;
+    if (k >= (o < m.maxbs ? sp.a1 : sp.b1)) continue;
     const double* r = con + C_STRIDE * c;
     int b1 = m.geom_body[(int)r[C_G1]], b2 = m.geom_body[(int)r[C_G2]];
     V3 p = ld3(r + C_POS);
@@ -85,9 +131,10 @@ __device__ int pgs_rows(const Tile<G>& T, const DModel& m, const WsLayout& w, co
       if (!hit[t]) continue;
       if (row < m.maxrows) {
         double* jr = J + row * nv;
-        for (int k = 0; k < nv; k++) jr[k] = 0.0;
-        jr[da] = t == 0 ? 1.0 : -1.0;
         double* rr = R + PR_STRIDE * row;
+        rr[PR_SPAN] = pack_span(m, m.dof_block[da], -1);
+        span_each(Span::of(rr[PR_SPAN]), [&](int k) { jr[k] = 0.0; });
+        jr[da] = t == 0 ? 1.0 : -1.0;
         rr[PR_KIND] = PK_NORMAL;
         rr[PR_SEP] = sep[t];
         rr[PR_MU] = 0.0;
@@ -109,7 +156,9 @@ __device__ int pgs_rows(const Tile<G>& T, const DModel& m, const WsLayout& w, co
     const double* c = m.eq_poly + 5 * q;
     double q1 = ws[w.qpos + m.jnt_qposadr[j1]] - m.qpos0[m.jnt_qposadr[j1]];
     double* jr = J + row * nv;
-    for (int k = 0; k < nv; k++) jr[k] = 0.0;
+    double* rr = R + PR_STRIDE * row;
+    rr[PR_SPAN] = pack_span(m, m.dof_block[m.jnt_dofadr[j1]], j2 != -1 ? m.dof_block[m.jnt_dofadr[j2]] : -1);
+    span_each(Span::of(rr[PR_SPAN]), [&](int k) { jr[k] = 0.0; });
     jr[m.jnt_dofadr[j1]] += 1.0;
     double poly = c[0];
     if (j2 != -1) {
@@ -117,7 +166,6 @@ __device__ int pgs_rows(const Tile<G>& T, const DModel& m, const WsLayout& w, co
       poly = c[0] + x * (c[1] + x * (c[2] + x * (c[3] + x * c[4])));
       jr[m.jnt_dofadr[j2]] -= c[1] + x * (2.0 * c[2] + x * (3.0 * c[3] + x * 4.0 * c[4]));
     }
-    double* rr = R + PR_STRIDE * row;
     rr[PR_KIND] = PK_BILATERAL;
     rr[PR_SEP] = q1 - poly;
     rr[PR_MU] = 0.0;
@@ -135,13 +183,12 @@ __device__ int pgs_rows(const Tile<G>& T, const DModel& m, const WsLayout& w, co
   return nr;
 }
 
-// x <- (L L')^-1 x for one right-hand side, by one lane, per dof block, with
-// the reference's operations (math.rs:451-463: row-oriented forward sweep
-// dividing by the pivot, then column-oriented backward sweep).
-__device__ inline void lane_mass_solve(const DModel& m, const double* L, double* x) {
-  int nv = m.nv;
-  for (int b = 0; b < m.nblock; b++) {
-    int s0 = m.block_adr[2 * b], s1 = m.block_adr[2 * b + 1];
+// x <- (L L')^-1 x for one right-hand side, by one lane, on the trees of a
+// span, with the reference's operations (math.rs:451-463: row-oriented forward
+// sweep dividing by the pivot, then column-oriented backward sweep).
+__device__ inline void lane_mass_solve(const Span& sp, int nv, const double* L, double* x) {
+  for (int t = 0; t < 2; t++) {
+    int s0 = t == 0 ? sp.a0 : sp.b0, s1 = t == 0 ? sp.a1 : sp.b1;
     for (int i = s0; i < s1; i++) x[i] = (x[i] - dot_ref(L + i * nv + s0, 1, x + s0, 1, i - s0)) / L[i * nv + i];
     for (int i = s1 - 1; i >= s0; i--) {
       x[i] /= L[i * nv + i];
@@ -179,10 +226,11 @@ __device__ __noinline__ int pgs_solve(const Tile<G>& T, const DModel& m, const W
   for (int r = lane; r < nr; r += G) {
     double* x = MJ + r * nv;
     const double* jr = J + r * nv;
-    for (int k = 0; k < nv; k++) x[k] = jr[k];
-    lane_mass_solve(m, L, x);
+    Span sp = Span::of(R[PR_STRIDE * r + PR_SPAN]);
+    span_each(sp, [&](int k) { x[k] = jr[k]; });
+    lane_mass_solve(sp, nv, L, x);
     double a = 0.0;
-    for (int k = 0; k < nv; k++) a += jr[k] * x[k];
+    span_each(sp, [&](int k) { a += jr[k] * x[k]; });
     R[PR_STRIDE * r + PR_INVA] = a > 1e-12 ? 1.0 / a : 0.0;
   }
   // warm start: the nearest previous contact of the same geom pair within
@@ -214,14 +262,47 @@ __device__ __noinline__ int pgs_solve(const Tile<G>& T, const DModel& m, const W
       R[PR_STRIDE * (3 * c + 2) + PR_LAMBDA] = dot(f, ld3(cr + C_T2));
     }
   }
+  // islands: trees joined by rows, each named by its lowest tree
+  int* tree = reinterpret_cast<int*>(e.ws + w.grad);  // [nblock] (free on this path)
+  for (int b = lane; b < m.nblock; b += G) tree[b] = b;
   T.sync();
-  for (int k = lane; k < nv; k += G) {
-    double vk = v[k];
-    for (int r = 0; r < nr; r++) {
-      double l = R[PR_STRIDE * r + PR_LAMBDA];
-      if (l != 0.0) vk += MJ[r * nv + k] * l;
+  for (bool more = m.nblock > 1; more;) {
+    bool changed = false;
+    for (int r = lane; r < nr; r += G) {
+      Span sp = Span::of(R[PR_STRIDE * r + PR_SPAN]);
+      if (sp.b1 == 0) continue;
+      int a = m.dof_block[sp.a0], b = m.dof_block[sp.b0];
+      int ta = tree[a], tb = tree[b];
+      if (ta != tb) {
+        atomicMin(tree + (ta > tb ? a : b), ta < tb ? ta : tb);
+        changed = true;
+      }
     }
-    v[k] = vk;
+    T.sync();
+    more = T.any(changed);
+  }
+  // the rows of each lane's islands, in row order (an island's lane: its
+  // rank among the islands, modulo the tile)
+  int* mine = reinterpret_cast<int*>(e.scr + s.isl_row);  // [maxrows] lists, then [maxrows] lanes of the rows
+  int* row_lane = mine + m.maxrows;
+  for (int r = lane; r < nr; r += G) {
+    Span sp = Span::of(R[PR_STRIDE * r + PR_SPAN]);
+    int t = sp.a1 > 0 ? tree[m.dof_block[sp.a0]] : 0, rank = 0;
+    for (int b = 0; b < t; b++) rank += tree[b] == b ? 1 : 0;
+    row_lane[r] = rank % G;
+  }
+  T.sync();
+  int count = 0;
+  for (int r = 0; r < nr; r++) count += row_lane[r] == lane ? 1 : 0;
+  int all;
+  int first = T.excl_scan(count, &all);
+  for (int r = 0, k = first; r < nr; r++)
+    if (row_lane[r] == lane) mine[k++] = r;
+  // the warm start's impulses
+  for (int x = first; x < first + count; x++) {
+    int r = mine[x];
+    double l = R[PR_STRIDE * r + PR_LAMBDA];
+    if (l != 0.0) span_each(Span::of(R[PR_STRIDE * r + PR_SPAN]), [&](int k) { v[k] += MJ[r * nv + k] * l; });
   }
   T.sync();
   // solver.rs:44-50
@@ -233,13 +314,24 @@ __device__ __noinline__ int pgs_solve(const Tile<G>& T, const DModel& m, const W
   // one Gauss-Seidel sweep; returns the largest velocity change
   auto sweep = [&](bool use_bias) -> double {
     double max_dv = 0.0;
-    for (int r = 0; r < nr; r++) {
+    int next = count > 0 ? mine[first] : 0;
+    for (int x = first; x < first + count; x++) {
+      const int r = next;
+      if (x + 1 < first + count) {
+        next = mine[x + 1];
+        prefetch_row(R + PR_STRIDE * next);
+        // (the span of the row after this one is most often this one's)
+        const int a0 = Span::of(R[PR_STRIDE * r + PR_SPAN]).a0;
+        prefetch_row(J + next * nv + a0);
+        prefetch_row(MJ + next * nv + a0);
+      }
       double* rr = R + PR_STRIDE * r;
       double inv_a = rr[PR_INVA];
       if (inv_a == 0.0) continue;
       const double* jr = J + r * nv;
+      const Span sp = Span::of(rr[PR_SPAN]);
       double jv = 0.0;
-      for (int k = 0; k < nv; k++) jv += jr[k] * v[k];
+      span_each(sp, [&](int k) { jv += jr[k] * v[k]; });
       double lam = rr[PR_LAMBDA];
       int kind = (int)rr[PR_KIND];
       double nw;
@@ -280,20 +372,19 @@ __device__ __noinline__ int pgs_solve(const Tile<G>& T, const DModel& m, const W
       double dl = nw - lam;
       if (dl != 0.0) {
         max_dv = fmax(max_dv, fabs(dl) / inv_a);
-        T.sync();  // every lane has read v and the impulses
         const double* mr = MJ + r * nv;
-        for (int k = lane; k < nv; k += G) v[k] += mr[k] * dl;
-        if (lane == 0) rr[PR_LAMBDA] = nw;
-        T.sync();
+        span_each(sp, [&](int k) { v[k] += mr[k] * dl; });
+        rr[PR_LAMBDA] = nw;
       }
     }
-    return max_dv;
+    return T.fmax(max_dv);
   };
   int sweeps = 0;
   for (int it = 0; it < m.iterations; it++) {
     sweeps++;
     if (sweep(true) < PGS_TOLERANCE) break;
   }
+  T.sync();
   for (int k = lane; k < nv; k += G) vpos[k] = v[k];
   T.sync();
   int nrelax = max(m.iterations / 3, 2);
@@ -301,6 +392,7 @@ __device__ __noinline__ int pgs_solve(const Tile<G>& T, const DModel& m, const W
     sweeps++;
     if (sweep(false) < PGS_TOLERANCE) break;
   }
+  T.sync();
   // this step's contacts and impulses for the next warm start
   for (int c = lane; c < nc; c += G) {
     const double* cr = con + C_STRIDE * c;

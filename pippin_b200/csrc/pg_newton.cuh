@@ -925,10 +925,223 @@ __device__ inline int newton_small(const Tile<G>& T, int k, int nr, const double
   return iters;
 }
 
+constexpr int TREE_N = 6;  // dofs of the trees a lane solves on its own (a free body)
+
+// The two sums of a line search step over an island's rows (or, with `gate`,
+// of the cost gate: the rows' costs at a0 and at the warm start, residuals in
+// R_JP and R_JAR).
+__device__ __forceinline__ double2 row_sums(const double* R, const int* rows, int cnt, double al, bool gate) {
+  double2 d{0.0, 0.0};
+#pragma unroll 2
+  for (int r = 0; r < cnt; r++) {
+    const double* rr = R + R_STRIDE * rows[r];
+    double e0 = rr[R_JP], e1 = rr[R_JAR], D = rr[R_D];
+    if (gate) {
+      if (row_active(rr, e0)) d.x += 0.5 * D * e0 * e0;
+      if (row_active(rr, e1)) d.y += 0.5 * D * e1 * e1;
+    } else {
+      double v = e1 + al * e0;
+      if (row_active(rr, v)) {
+        double dq = D * e0;
+        d.x += dq * v;
+        d.y += dq * e0;
+      }
+    }
+  }
+  return d;
+}
+
+// newton.rs:224-371 by one lane for an island of one tree: dofs [s0, s0 + n),
+// n <= TREE_N, rows rows[0, cnt) of J / R in order (one tree's columns of J at
+// s0). M, the Hessian and its factor stay in registers, the rows' residuals in
+// their records. Sums run in newton_dense's order but for the line search's.
+// Adds the constraint force to qfrc, leaves the solution in a; returns the
+// iteration count.
+__device__ __noinline__ inline int newton_tree(int nv, int s0, int n, const int* rows, int cnt, const double* J, double* R,
+                                               const double* M, double* a, const double* warm, int max_iters, double tol,
+                                               double* qfrc) {
+  double mm[TREE_N * (TREE_N + 1) / 2], a0[TREE_N], x[TREE_N], y[TREE_N];
+  auto at = [](int i, int j) { return i * (i + 1) / 2 + j; };
+#pragma unroll
+  for (int i = 0; i < TREE_N; i++) {
+#pragma unroll
+    for (int j = 0; j <= i; j++) mm[at(i, j)] = i < n ? M[(s0 + i) * nv + s0 + j] : (i == j ? 1.0 : 0.0);
+    x[i] = a0[i] = i < n ? a[s0 + i] : 0.0;
+  }
+  auto mul = [&](const double (&u)[TREE_N], double (&o)[TREE_N]) {
+#pragma unroll
+    for (int i = 0; i < TREE_N; i++) {
+      double t = 0.0;
+#pragma unroll
+      for (int j = 0; j < TREE_N; j++) t += mm[i >= j ? at(i, j) : at(j, i)] * u[j];
+      o[i] = t;
+    }
+  };
+  // f(record, row's entries) for every row, the next row's loads under way
+  auto each = [&](auto f) {
+    double j[TREE_N];
+    const double* p = J + rows[0] * nv + s0;
+#pragma unroll
+    for (int i = 0; i < TREE_N; i++) j[i] = i < n ? p[i] : 0.0;
+#pragma unroll 1
+    for (int t = 0; t < cnt; t++) {
+      double nj[TREE_N];
+      p = J + rows[t + 1 < cnt ? t + 1 : t] * nv + s0;
+#pragma unroll
+      for (int i = 0; i < TREE_N; i++) nj[i] = i < n ? p[i] : 0.0;
+      f(R + R_STRIDE * rows[t], j);
+#pragma unroll
+      for (int i = 0; i < TREE_N; i++) j[i] = nj[i];
+    }
+  };
+  // over the dofs in the order of a tile's sum
+  auto sum = [](const double (&u)[TREE_N], const double (&v)[TREE_N]) {
+    auto w = [&](int i) { return __dmul_rn(u[i], v[i]); };
+    return ((w(0) + w(4)) + w(2)) + ((w(1) + w(5)) + w(3));
+  };
+  auto dot = [](const double (&u)[TREE_N], const double (&v)[TREE_N]) {
+    double t = 0.0;
+#pragma unroll
+    for (int i = 0; i < TREE_N; i++) t += u[i] * v[i];
+    return t;
+  };
+  if (warm) {
+    double w[TREE_N], d[TREE_N];
+#pragma unroll
+    for (int i = 0; i < TREE_N; i++) {
+      w[i] = i < n ? warm[s0 + i] : 0.0;
+      d[i] = w[i] - a0[i];
+    }
+    mul(d, y);
+    each([&](double* rr, const double(&j)[TREE_N]) {
+      rr[R_JP] = dot(j, a0) - rr[R_AREF];
+      rr[R_JAR] = dot(j, w) - rr[R_AREF];
+    });
+    double2 c = row_sums(R, rows, cnt, 0.0, true);
+    if (0.5 * sum(d, y) + c.y < c.x) {
+#pragma unroll
+      for (int i = 0; i < TREE_N; i++) x[i] = w[i];
+    }
+  }
+  mul(a0, y);
+  const double scale = 1.0 + sqrt(sum(y, y));
+  int iters = 0;
+  const int maxit = max_iters > 1 ? max_iters : 1;
+  double f[TREE_N];
+#pragma unroll 1
+  while (true) {
+    // gradient, active set and H = M + J_A' D J_A in one pass over the rows
+    double t[TREE_N], g[TREE_N], h[TREE_N * (TREE_N + 1) / 2];
+#pragma unroll
+    for (int i = 0; i < TREE_N; i++) {
+      t[i] = x[i] - a0[i];
+      f[i] = 0.0;
+    }
+    mul(t, g);
+#pragma unroll
+    for (int k = 0; k < TREE_N * (TREE_N + 1) / 2; k++) h[k] = mm[k];
+    bool same = true;
+    each([&](double* rr, const double(&j)[TREE_N]) {
+      double jar = dot(j, x) - rr[R_AREF];
+      rr[R_JAR] = jar;
+      double act = row_active(rr, jar) ? 1.0 : 0.0;
+      if (act != rr[R_ACT]) same = false;
+      rr[R_ACT] = act;
+      if (act != 0.0) {
+        double D = rr[R_D], dj = D * jar;
+#pragma unroll
+        for (int i = 0; i < TREE_N; i++) {
+          f[i] += dj * j[i];
+          g[i] += dj * j[i];
+          double e = D * j[i];
+#pragma unroll
+          for (int k = 0; k <= i; k++) h[at(i, k)] += e * j[k];
+        }
+      }
+    });
+    if (iters >= maxit) break;  // f is the force at the last step's end
+    iters++;
+    if (sqrt(sum(g, g)) < tol * scale || (cnt <= 128 && same && iters > 1)) break;
+    // p = -H^-1 g, by the steps of chol_left and solve_left
+    bool ok = true;
+    double p[TREE_N], ri[TREE_N];
+#pragma unroll
+    for (int k = 0; k < TREE_N; k++) {
+#pragma unroll
+      for (int i = k; i < TREE_N; i++) {
+        double u = 0.0;
+#pragma unroll
+        for (int q = 0; q < k; q++) u += h[at(i, q)] * h[at(k, q)];
+        double d = h[at(i, k)] - u;
+        if (i == k) {
+          ok = ok && d > 0.0;
+          ri[k] = rsqrt(d);
+        } else {
+          h[at(i, k)] = d * ri[k];
+        }
+      }
+    }
+    if (!ok) break;
+#pragma unroll
+    for (int i = 0; i < TREE_N; i++) {
+      double u = -g[i];
+#pragma unroll
+      for (int q = 0; q < i; q++) u -= h[at(i, q)] * p[q];
+      p[i] = u * ri[i];
+    }
+#pragma unroll
+    for (int i = TREE_N - 1; i >= 0; i--) {
+      double u = p[i];
+#pragma unroll
+      for (int q = TREE_N - 1; q > i; q--) u -= h[at(q, i)] * p[q];
+      p[i] = u * ri[i];
+    }
+    // exact line search on the piecewise quadratic along p
+    mul(p, y);
+    const double mpp = sum(p, y), mpg = sum(t, y);
+    each([&](double* rr, const double(&j)[TREE_N]) { rr[R_JP] = dot(j, p); });
+    double lo = 0.0, hi = INFINITY, al = 0.0, ltol = 0.0;
+#pragma unroll 1
+    for (int it = -1; it < 50; it++) {
+      double2 d = row_sums(R, rows, cnt, al, false);
+      double d1 = (al * mpp + mpg) + d.x, d2 = mpp + d.y;
+      if (it < 0) {
+        ltol = 1e-12 * fmax(fabs(d1), 1e-30);
+        al = 1.0;
+        continue;
+      }
+      if (fabs(d1) <= ltol) break;
+      if (d1 < 0.0) lo = al;
+      else hi = al;
+      double next = al - d1 / fmax(d2, 1e-30);
+      if (next <= lo || next >= hi) next = isfinite(hi) ? 0.5 * (lo + hi) : 2.0 * fmax(al, lo);
+      bool end = fabs(next - al) <= 1e-14 * fmax(fabs(al), 1.0);
+      al = next;
+      if (end) break;
+    }
+#pragma unroll
+    for (int i = 0; i < TREE_N; i++) x[i] += al * p[i];
+  }
+#pragma unroll
+  for (int i = 0; i < TREE_N; i++)
+    if (i < n) {
+      a[s0 + i] = x[i];
+      qfrc[s0 + i] -= f[i];
+    }
+  return iters;
+}
+
 // newton.rs:391-473 for models with several dof blocks: islands are the
-// blocks joined by rows touching more than one; each is solved as its own
-// dense subproblem (in place when one island spans every block).
-template <int G>
+// blocks joined by rows touching more than one. An island of one small tree
+// (a body on the floor, the common one) is a lane's own solve, all of them
+// side by side; the others are solved one after another on the whole tile as
+// dense subproblems (in place when one island spans every block). LANES =
+// false leaves every island to the tile (the learned start's candidate is
+// formed there). What bounds a tile on a 6 x 6 system is its syncs and the 26
+// idle lanes: with every island on the tile in turn, 4096 envs of 8 hulls took
+// 1541 us in this phase (62k warp instructions an env), the tabletop 778 us;
+// now 615 and 348.
+template <int G, bool LANES>
 __device__ __noinline__ int newton_islands(const Tile<G>& T, const DModel& m, const WsLayout& w, const ScrLayout& s,
                                            const EnvCtx& e, int nr, double* a, const double* warm,
                                            const NewtonBufs& B, bool cand) {
@@ -950,31 +1163,30 @@ __device__ __noinline__ int newton_islands(const Tile<G>& T, const DModel& m, co
     rmask[r] = mk;
   }
   T.sync();
-  if (lane == 0) {
-    int par[64];
-    for (int b = 0; b < m.nblock; b++) par[b] = b;
-    auto find = [&](int x) {
-      while (par[x] != x) {
-        par[x] = par[par[x]];
-        x = par[x];
-      }
-      return x;
-    };
-    for (int r = 0; r < nr; r++) {
+  // each block's island is the lowest block it is joined to
+  int* tree = reinterpret_cast<int*>(ws + w.grad);  // [nblock] (free until the solves)
+  for (int b = lane; b < m.nblock; b += G) tree[b] = b;
+  T.sync();
+  for (bool more = true; more;) {
+    bool changed = false;
+    for (int r = lane; r < nr; r += G) {
       unsigned long long mk = rmask[r];
-      if (!mk) continue;
-      int first = __ffsll((long long)mk) - 1;
-      mk &= mk - 1;
-      while (mk) {
-        int b = __ffsll((long long)mk) - 1;
-        mk &= mk - 1;
-        int x = find(first), y = find(b);
-        if (x != y) par[x > y ? x : y] = x < y ? x : y;
+      if (!(mk & (mk - 1))) continue;  // no block or one
+      int low = m.nblock;
+      for (unsigned long long q = mk; q; q &= q - 1) low = min(low, tree[__ffsll((long long)q) - 1]);
+      for (unsigned long long q = mk; q; q &= q - 1) {
+        int b = __ffsll((long long)q) - 1;
+        if (tree[b] != low) {
+          atomicMin(tree + b, low);
+          changed = true;
+        }
       }
     }
-    for (int b = 0; b < m.nblock; b++) blk_isl[b] = find(b);
-    for (int r = 0; r < nr; r++) iscr[r] = rmask[r] ? blk_isl[__ffsll((long long)rmask[r]) - 1] : -1;
+    T.sync();
+    more = T.any(changed);
   }
+  for (int b = lane; b < m.nblock; b += G) blk_isl[b] = tree[b];
+  for (int r = lane; r < nr; r += G) iscr[r] = rmask[r] ? tree[__ffsll((long long)rmask[r]) - 1] : -1;
   T.sync();
   // islands in increasing id order; single island spanning all blocks -> in place
   int n_isl = 0, only = -1;
@@ -994,6 +1206,41 @@ __device__ __noinline__ int newton_islands(const Tile<G>& T, const DModel& m, co
     return it;
   }
   int iters = 0;
+  unsigned long long own = 0;  // islands of one small tree: solved by a lane each
+  if constexpr (LANES) {
+    unsigned long long joined = 0;
+    for (int b = 0; b < m.nblock; b++)
+      if (tree[b] != b) joined |= 1ull << tree[b];
+    for (int b = 0; b < m.nblock; b++)
+      if (tree[b] == b && !(joined >> b & 1ull) && m.block_adr[2 * b + 1] - m.block_adr[2 * b] <= TREE_N) own |= 1ull << b;
+    // lane l takes the islands l, l + G, ... of these, all lanes side by
+    // side; an island's rows are listed in row order
+    int* list = (int*)(e.scr + s.isl_row) + 2 * m.maxrows;  // after rmask words: [maxrows]
+    const int nown = __popcll(own);
+    for (int base = 0; base < nown; base += G) {
+      int isl = -1;
+      if (base + lane < nown) {
+        unsigned long long q = own;
+        for (int k = base + lane; k > 0; k--) q &= q - 1;
+        isl = __ffsll((long long)q) - 1;
+      }
+      int cnt = 0;
+      for (int r = 0; r < nr; r++) cnt += isl >= 0 && iscr[r] == isl ? 1 : 0;
+      int all;
+      int* rows = list + T.excl_scan(cnt, &all);
+      for (int r = 0, k = 0; k < cnt; r++)
+        if (iscr[r] == isl) rows[k++] = r;
+      if (cnt > 0) {
+        int s0 = m.block_adr[2 * isl];
+        int it = newton_tree(nv, s0, m.block_adr[2 * isl + 1] - s0, rows, cnt, J, R, e.qm, a, warm, max_iters, tol, qfrc);
+        iters = it > iters ? it : iters;
+      }
+      T.sync();
+    }
+    T.sync();
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) iters = max(iters, T.t.shfl_xor(iters, o));
+  }
   double* subM = e.scr + s.sub_m;
   double* subJ = e.scr + s.sub_j;
   double* subR = e.scr + s.sub_rows;
@@ -1001,6 +1248,7 @@ __device__ __noinline__ int newton_islands(const Tile<G>& T, const DModel& m, co
   double* suba = ws + w.vel;   // free until the solve returns
   double* wsub = ws + w.warm;  // gathered warm start
   for (int isl = 0; isl < m.nblock; isl++) {
+    if (own >> isl & 1ull) continue;
     bool has = false;
     for (int r = lane; r < nr; r += G) has |= iscr[r] == isl;
     if (!T.any(has)) continue;
@@ -1098,7 +1346,7 @@ __device__ int newton_solve(const Tile<G>& T, const DModel& m, const WsLayout& w
   T.sync();
   NewtonBufs B{ws + w.a0, ws + w.grad, ws + w.p, ws + w.tmp, ws + w.tmp2, ws + w.mp, e.fac, ws + w.rinv};
   if (m.nblock > 1) {
-    int it = newton_islands(T, m, w, s, e, nr, a, warm, B, cand);
+    int it = newton_islands<G, !LEARN>(T, m, w, s, e, nr, a, warm, B, cand);
     if (learned && ldump) dump_row_forces(T, nv, J, R, a, 4 * lnum, ldump);
     return it;
   }

@@ -311,72 +311,113 @@ __device__ __noinline__ int pgs_solve(const Tile<G>& T, const DModel& m, const W
   double a2 = h * omega * a1;
   double a3 = 1.0 / (1.0 + a2);
   double bias_rate = omega / a1, mass_scale = a2 * a3, impulse_scale = a3;
-  // one Gauss-Seidel sweep; returns the largest velocity change
+  // a row's new impulse from its J . v (solver.rs:164-215)
+  auto impulse = [&](const double* rr, int kind, double jv, double lam, double inv_a, double normal, bool use_bias) {
+    if (kind == PK_FRICTION) {
+      double bound = rr[PR_MU] * normal;
+      return fmin(fmax(lam - inv_a * jv, -bound), bound);
+    }
+    double bias = 0.0, ms = 1.0, is = 0.0;
+    if (kind == PK_NORMAL) {
+      double sl = rr[PR_SEP] + m.slop;
+      if (sl > 0.0) {
+        bias = sl / h;
+      } else if (use_bias) {
+        bias = fmax(bias_rate * sl, -PGS_MAX_BIAS_VELOCITY);
+        ms = mass_scale;
+        is = impulse_scale;
+      }
+      double delta = -inv_a * ms * (jv + bias) - is * lam;
+      return fmax(lam + delta, 0.0);
+    }
+    if (use_bias) {
+      bias = fmin(fmax(bias_rate * rr[PR_SEP], -PGS_MAX_BIAS_VELOCITY), PGS_MAX_BIAS_VELOCITY);
+      ms = mass_scale;
+      is = impulse_scale;
+    }
+    return lam - inv_a * ms * (jv + bias) - is * lam;
+  };
+  // one Gauss-Seidel sweep; returns the largest velocity change. The
+  // velocities of the tree that the last rows touched stay in registers (u,
+  // dofs [held, held + 6)), a contact's normal impulse with them; a row of two
+  // trees, or of a tree of more than six dofs, goes through shared memory.
   auto sweep = [&](bool use_bias) -> double {
     double max_dv = 0.0;
+    constexpr int NU = 6;
+    double u[NU];
+    int held = -1, hold_n = 0, normal_row = -1;
+    double normal_l = 0.0;
+    auto drop = [&]() {
+      if (held >= 0)
+#pragma unroll
+        for (int k = 0; k < NU; k++)
+          if (k < hold_n) v[held + k] = u[k];
+      held = -1;
+    };
     int next = count > 0 ? mine[first] : 0;
     for (int x = first; x < first + count; x++) {
       const int r = next;
+      double* rr = R + PR_STRIDE * r;
+      const double inv_a = rr[PR_INVA], lam = rr[PR_LAMBDA];
+      const Span sp = Span::of(rr[PR_SPAN]);
+      const int kind = (int)rr[PR_KIND];
       if (x + 1 < first + count) {
         next = mine[x + 1];
         prefetch_row(R + PR_STRIDE * next);
-        // (the span of the row after this one is most often this one's)
-        const int a0 = Span::of(R[PR_STRIDE * r + PR_SPAN]).a0;
-        prefetch_row(J + next * nv + a0);
-        prefetch_row(MJ + next * nv + a0);
+        // (the row after this one is most often of the same tree)
+        prefetch_row(J + next * nv + sp.a0);
+        prefetch_row(MJ + next * nv + sp.a0);
       }
-      double* rr = R + PR_STRIDE * r;
-      double inv_a = rr[PR_INVA];
       if (inv_a == 0.0) continue;
       const double* jr = J + r * nv;
-      const Span sp = Span::of(rr[PR_SPAN]);
-      double jv = 0.0;
-      span_each(sp, [&](int k) { jv += jr[k] * v[k]; });
-      double lam = rr[PR_LAMBDA];
-      int kind = (int)rr[PR_KIND];
-      double nw;
-      if (kind == PK_NORMAL) {
-        double sl = rr[PR_SEP] + m.slop;
-        double bias, ms, is;
-        if (sl > 0.0) {
-          bias = sl / h;
-          ms = 1.0;
-          is = 0.0;
-        } else if (use_bias) {
-          bias = fmax(bias_rate * sl, -PGS_MAX_BIAS_VELOCITY);
-          ms = mass_scale;
-          is = impulse_scale;
-        } else {
-          bias = 0.0;
-          ms = 1.0;
-          is = 0.0;
-        }
-        double delta = -inv_a * ms * (jv + bias) - is * lam;
-        nw = fmax(lam + delta, 0.0);
-      } else if (kind == PK_BILATERAL) {
-        double bias, ms, is;
-        if (use_bias) {
-          bias = fmin(fmax(bias_rate * rr[PR_SEP], -PGS_MAX_BIAS_VELOCITY), PGS_MAX_BIAS_VELOCITY);
-          ms = mass_scale;
-          is = impulse_scale;
-        } else {
-          bias = 0.0;
-          ms = 1.0;
-          is = 0.0;
-        }
-        nw = lam - inv_a * ms * (jv + bias) - is * lam;
-      } else {
-        double bound = rr[PR_MU] * R[PR_STRIDE * (int)rr[PR_NORMAL] + PR_LAMBDA];
-        nw = fmin(fmax(lam - inv_a * jv, -bound), bound);
+      const double* mr = MJ + r * nv;
+      double normal = 0.0;
+      if (kind == PK_FRICTION) {
+        int nrow = (int)rr[PR_NORMAL];
+        normal = nrow == normal_row ? normal_l : R[PR_STRIDE * nrow + PR_LAMBDA];
       }
-      double dl = nw - lam;
+      double nw, dl;
+      const int na = sp.a1 - sp.a0;
+      if (sp.b1 == 0 && na <= NU) {
+        if (held != sp.a0) {
+          drop();
+          held = sp.a0;
+          hold_n = na;
+#pragma unroll
+          for (int k = 0; k < NU; k++) u[k] = k < na ? v[sp.a0 + k] : 0.0;
+        }
+        double j[NU], w[NU];
+#pragma unroll
+        for (int k = 0; k < NU; k++) {
+          j[k] = k < na ? jr[sp.a0 + k] : 0.0;
+          w[k] = k < na ? mr[sp.a0 + k] : 0.0;
+        }
+        double jv = 0.0;
+#pragma unroll
+        for (int k = 0; k < NU; k++) jv += j[k] * u[k];
+        nw = impulse(rr, kind, jv, lam, inv_a, normal, use_bias);
+        dl = nw - lam;
+        if (dl != 0.0)
+#pragma unroll
+          for (int k = 0; k < NU; k++) u[k] += w[k] * dl;
+      } else {
+        drop();
+        double jv = 0.0;
+        span_each(sp, [&](int k) { jv += jr[k] * v[k]; });
+        nw = impulse(rr, kind, jv, lam, inv_a, normal, use_bias);
+        dl = nw - lam;
+        if (dl != 0.0) span_each(sp, [&](int k) { v[k] += mr[k] * dl; });
+      }
+      if (kind == PK_NORMAL) {
+        normal_row = r;
+        normal_l = nw;
+      }
       if (dl != 0.0) {
         max_dv = fmax(max_dv, fabs(dl) / inv_a);
-        const double* mr = MJ + r * nv;
-        span_each(sp, [&](int k) { v[k] += mr[k] * dl; });
         rr[PR_LAMBDA] = nw;
       }
     }
+    drop();
     return T.fmax(max_dv);
   };
   int sweeps = 0;

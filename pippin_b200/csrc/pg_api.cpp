@@ -609,7 +609,7 @@ void layouts(const HostModel& m, int maxcon, int maxrows, bool lane, WsLayout* w
   s->chol = take(nv * nv);
   int multi = m.dof_blocks.size() / 2 > 1;
   s->sub_m = take(multi ? nv * nv : 0);
-  s->sub_j = take(multi ? maxrows * nv : 0);
+  s->sub_j = take(multi ? maxrows * nv + 16 : 0);  // (16: PGS aligns its rows' lines in it)
   s->sub_rows = take(multi ? maxrows * R_STRIDE : 0);
   s->isl_dof = take(nv + 2);
   s->isl_row = take(maxrows + (nv + maxrows + 1) / 2 + 2);

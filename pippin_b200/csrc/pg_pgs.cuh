@@ -11,10 +11,12 @@
 // joined by rows) share no velocity, so each lane sweeps islands of its own, in
 // row order, and the tile meets once a sweep for the largest change: the
 // sequential sweep's result to the bit (a sum's terms that are left out are
-// zero). Impulses live in the row records. With the whole tile on one row at a
-// time (48 dofs a product, two tile syncs a row) 1001 envs of 8 hulls took
-// 6.67 ms in this phase, now 1.43 ms; what bounds it now is the
-// latency of the row's loads, which are prefetched a row ahead.
+// zero). With the whole tile on one row at a time (48 dofs a product, two tile
+// syncs a row) 1001 envs of 8 hulls took 6.67 ms in this phase; islands side by
+// side 1.43 ms, and with a row's numbers in one 128-byte line, prefetched a row
+// ahead, and the tree's velocities in registers 1.17 ms (32 lanes an env, from
+// a state without impulses). What bounds it now is the chain of one row's loads
+// and sums after another.
 #pragma once
 #include "pg_newton.cuh"
 
@@ -298,6 +300,33 @@ __device__ __noinline__ int pgs_solve(const Tile<G>& T, const DModel& m, const W
   int first = T.excl_scan(count, &all);
   for (int r = 0, k = first; r < nr; r++)
     if (row_lane[r] == lane) mine[k++] = r;
+  // rows of one tree of at most six dofs, one 128-byte line each in the order
+  // of the lists: J, M^-1 J', 1 / a, impulse, sep or mu, kind (a sweep reads
+  // one line a row instead of parts of seven sectors)
+  constexpr int NU = 6;
+  enum { L_J = 0, L_W = NU, L_INVA = 2 * NU, L_LAMBDA, L_ARG, L_KIND, L_STRIDE };
+  static_assert(L_STRIDE == 16, "a line a row");
+  const bool lines = m.nblock > 1 && nv >= L_STRIDE;  // (the island buffer, unused on this path, holds them)
+  double* line = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(e.scr + s.sub_j) + 127) & ~uintptr_t(127));
+  // a line's kind: the row's, plus 4 when the row goes another way
+  if (lines)
+    for (int x = first; x < first + count; x++) {
+      const int r = mine[x];
+      const double* rr = R + PR_STRIDE * r;
+      const Span sp = Span::of(rr[PR_SPAN]);
+      double* o = line + L_STRIDE * x;
+      const int na = sp.a1 - sp.a0;
+      const bool fits = sp.b1 == 0 && na <= NU;
+      for (int k = 0; k < NU; k++) {
+        o[L_J + k] = fits && k < na ? J[r * nv + sp.a0 + k] : 0.0;
+        o[L_W + k] = fits && k < na ? MJ[r * nv + sp.a0 + k] : 0.0;
+      }
+      o[L_INVA] = rr[PR_INVA];
+      o[L_LAMBDA] = rr[PR_LAMBDA];
+      o[L_ARG] = rr[PR_KIND] == PK_FRICTION ? rr[PR_MU] : rr[PR_SEP];
+      // (span start in the upper part)
+      o[L_KIND] = rr[PR_KIND] + (fits ? 0.0 : 4.0) + 8.0 * sp.a0 + 1024.0 * na;
+    }
   // the warm start's impulses
   for (int x = first; x < first + count; x++) {
     int r = mine[x];
@@ -312,14 +341,15 @@ __device__ __noinline__ int pgs_solve(const Tile<G>& T, const DModel& m, const W
   double a3 = 1.0 / (1.0 + a2);
   double bias_rate = omega / a1, mass_scale = a2 * a3, impulse_scale = a3;
   // a row's new impulse from its J . v (solver.rs:164-215)
-  auto impulse = [&](const double* rr, int kind, double jv, double lam, double inv_a, double normal, bool use_bias) {
+  // (arg: the row's mu or separation)
+  auto impulse = [&](double arg, int kind, double jv, double lam, double inv_a, double normal, bool use_bias) {
     if (kind == PK_FRICTION) {
-      double bound = rr[PR_MU] * normal;
+      double bound = arg * normal;
       return fmin(fmax(lam - inv_a * jv, -bound), bound);
     }
     double bias = 0.0, ms = 1.0, is = 0.0;
     if (kind == PK_NORMAL) {
-      double sl = rr[PR_SEP] + m.slop;
+      double sl = arg + m.slop;
       if (sl > 0.0) {
         bias = sl / h;
       } else if (use_bias) {
@@ -331,7 +361,7 @@ __device__ __noinline__ int pgs_solve(const Tile<G>& T, const DModel& m, const W
       return fmax(lam + delta, 0.0);
     }
     if (use_bias) {
-      bias = fmin(fmax(bias_rate * rr[PR_SEP], -PGS_MAX_BIAS_VELOCITY), PGS_MAX_BIAS_VELOCITY);
+      bias = fmin(fmax(bias_rate * arg, -PGS_MAX_BIAS_VELOCITY), PGS_MAX_BIAS_VELOCITY);
       ms = mass_scale;
       is = impulse_scale;
     }
@@ -343,9 +373,8 @@ __device__ __noinline__ int pgs_solve(const Tile<G>& T, const DModel& m, const W
   // trees, or of a tree of more than six dofs, goes through shared memory.
   auto sweep = [&](bool use_bias) -> double {
     double max_dv = 0.0;
-    constexpr int NU = 6;
     double u[NU];
-    int held = -1, hold_n = 0, normal_row = -1;
+    int held = -1, hold_n = 0;
     double normal_l = 0.0;
     auto drop = [&]() {
       if (held >= 0)
@@ -354,68 +383,72 @@ __device__ __noinline__ int pgs_solve(const Tile<G>& T, const DModel& m, const W
           if (k < hold_n) v[held + k] = u[k];
       held = -1;
     };
-    int next = count > 0 ? mine[first] : 0;
     for (int x = first; x < first + count; x++) {
-      const int r = next;
-      double* rr = R + PR_STRIDE * r;
-      const double inv_a = rr[PR_INVA], lam = rr[PR_LAMBDA];
-      const Span sp = Span::of(rr[PR_SPAN]);
-      const int kind = (int)rr[PR_KIND];
-      if (x + 1 < first + count) {
-        next = mine[x + 1];
-        prefetch_row(R + PR_STRIDE * next);
-        // (the row after this one is most often of the same tree)
-        prefetch_row(J + next * nv + sp.a0);
-        prefetch_row(MJ + next * nv + sp.a0);
+      double* o = line + L_STRIDE * x;
+      double inv_a, lam, arg;
+      int kind, a0 = 0, na = 0, r = -1;
+      Span sp{0, 0, 0, 0};
+      bool fits = false;
+      if (lines) {
+        if (x + 1 < first + count) prefetch_row(o + L_STRIDE);
+        inv_a = o[L_INVA];
+        lam = o[L_LAMBDA];
+        arg = o[L_ARG];
+        const int code = (int)o[L_KIND];
+        kind = code & 3;
+        fits = !(code & 4);
+        a0 = code >> 3 & 127;
+        na = code >> 10;
       }
-      if (inv_a == 0.0) continue;
-      const double* jr = J + r * nv;
-      const double* mr = MJ + r * nv;
-      double normal = 0.0;
-      if (kind == PK_FRICTION) {
-        int nrow = (int)rr[PR_NORMAL];
-        normal = nrow == normal_row ? normal_l : R[PR_STRIDE * nrow + PR_LAMBDA];
+      if (!fits) {
+        r = mine[x];
+        const double* rr = R + PR_STRIDE * r;
+        inv_a = rr[PR_INVA];
+        lam = rr[PR_LAMBDA];
+        sp = Span::of(rr[PR_SPAN]);
+        kind = (int)rr[PR_KIND];
+        arg = kind == PK_FRICTION ? rr[PR_MU] : rr[PR_SEP];
       }
+      if (inv_a == 0.0) {
+        if (kind == PK_NORMAL) normal_l = lam;
+        continue;
+      }
+      // a contact's normal row stands before its friction rows in the list
+      const double normal = kind == PK_FRICTION ? normal_l : 0.0;
       double nw, dl;
-      const int na = sp.a1 - sp.a0;
-      if (sp.b1 == 0 && na <= NU) {
-        if (held != sp.a0) {
+      if (fits) {
+        if (held != a0) {
           drop();
-          held = sp.a0;
+          held = a0;
           hold_n = na;
 #pragma unroll
-          for (int k = 0; k < NU; k++) u[k] = k < na ? v[sp.a0 + k] : 0.0;
-        }
-        double j[NU], w[NU];
-#pragma unroll
-        for (int k = 0; k < NU; k++) {
-          j[k] = k < na ? jr[sp.a0 + k] : 0.0;
-          w[k] = k < na ? mr[sp.a0 + k] : 0.0;
+          for (int k = 0; k < NU; k++) u[k] = k < na ? v[a0 + k] : 0.0;
         }
         double jv = 0.0;
 #pragma unroll
-        for (int k = 0; k < NU; k++) jv += j[k] * u[k];
-        nw = impulse(rr, kind, jv, lam, inv_a, normal, use_bias);
+        for (int k = 0; k < NU; k++) jv += o[L_J + k] * u[k];
+        nw = impulse(arg, kind, jv, lam, inv_a, normal, use_bias);
         dl = nw - lam;
-        if (dl != 0.0)
+        if (dl != 0.0) {
 #pragma unroll
-          for (int k = 0; k < NU; k++) u[k] += w[k] * dl;
+          for (int k = 0; k < NU; k++) u[k] += o[L_W + k] * dl;
+          o[L_LAMBDA] = nw;
+        }
       } else {
         drop();
+        const double* jr = J + r * nv;
+        const double* mr = MJ + r * nv;
         double jv = 0.0;
         span_each(sp, [&](int k) { jv += jr[k] * v[k]; });
-        nw = impulse(rr, kind, jv, lam, inv_a, normal, use_bias);
+        nw = impulse(arg, kind, jv, lam, inv_a, normal, use_bias);
         dl = nw - lam;
-        if (dl != 0.0) span_each(sp, [&](int k) { v[k] += mr[k] * dl; });
+        if (dl != 0.0) {
+          span_each(sp, [&](int k) { v[k] += mr[k] * dl; });
+          R[PR_STRIDE * r + PR_LAMBDA] = nw;
+        }
       }
-      if (kind == PK_NORMAL) {
-        normal_row = r;
-        normal_l = nw;
-      }
-      if (dl != 0.0) {
-        max_dv = fmax(max_dv, fabs(dl) / inv_a);
-        rr[PR_LAMBDA] = nw;
-      }
+      if (kind == PK_NORMAL) normal_l = nw;
+      if (dl != 0.0) max_dv = fmax(max_dv, fabs(dl) / inv_a);
     }
     drop();
     return T.fmax(max_dv);
@@ -433,6 +466,9 @@ __device__ __noinline__ int pgs_solve(const Tile<G>& T, const DModel& m, const W
     sweeps++;
     if (sweep(false) < PGS_TOLERANCE) break;
   }
+  if (lines)
+    for (int x = first; x < first + count; x++)
+      if (!((int)line[L_STRIDE * x + L_KIND] & 4)) R[PR_STRIDE * mine[x] + PR_LAMBDA] = line[L_STRIDE * x + L_LAMBDA];
   T.sync();
   // this step's contacts and impulses for the next warm start
   for (int c = lane; c < nc; c += G) {

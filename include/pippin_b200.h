@@ -233,8 +233,10 @@ int pg_debug_forward(pg_handle* h, int64_t env, double* qm, double* qfrc_bias, d
 int pg_invweight(pg_handle* h, int64_t env, double* body, double* dof);
 
 /* Launch shape: lanes per env (8, 16, 32) and envs per block; 0 = keep.
- * pg_autotune times the candidate shapes on the current state (which it
- * saves and restores) and keeps the fastest. */
+ * Naming a shape makes pg_step run the phase kernels in it where it would run
+ * the substep in one kernel. pg_autotune times the candidate shapes on the
+ * current state (which it saves and restores) and keeps the fastest; it has
+ * nothing to do for a handle whose substep is one kernel. */
 int pg_set_launch(pg_handle* h, int lanes_per_env, int envs_per_block);
 int pg_get_launch(const pg_handle* h, int* lanes_per_env, int* envs_per_block, int* blocks);
 int pg_autotune(pg_handle* h, int64_t nstep);

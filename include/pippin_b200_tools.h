@@ -30,6 +30,12 @@ int pg_time_phases(pg_handle* h, int64_t start, int64_t end, int64_t nstep, cons
  * Returns PG_OK or PG_ERR_INVALID. */
 int pg_phase_launch(const pg_handle* h, int phase, int* lanes_per_env, int* envs_per_block, int* blocks);
 
+/* Lanes per env of the kernel that pg_step's substeps run in with the
+ * handle's current solver settings and launch shape: 1 or 4 (the whole substep
+ * in one kernel, csrc/pg_lane.cu and pg_quad.cu), or 0 for the three phase
+ * kernels. pg_time_phases always runs the phase kernels. -1: NULL handle. */
+int pg_step_lanes(const pg_handle* h);
+
 /* How many Newton-phase tiles pg_step_static runs at once out of its fixed
  * scratch array, for tiles of `tile_bytes` and blocks of `tiles_per_block`
  * tiles (a whole number of blocks; the envs beyond them follow in turn).

@@ -66,6 +66,7 @@ SIGNATURES = [
     ("pg_fp64_peak", _i32, [_i32, _i32, _pd, _pd]),
     ("pg_time_phases", _i32, [_vp, _i64, _i64, _i64, _vp, _pf]),
     ("pg_phase_launch", _i32, [_vp, _i32, _pi32, _pi32, _pi32]),
+    ("pg_step_lanes", _i32, [_vp]),
     ("pg_static_tiles", _i32, [_sz, _i32, _pi64]),
     ("pg_hull_support", _i32, [_vp, _i32, _pd, _i64, _pi32]),
     ("pg_set_warm_mlp", _i32, [_vp, _pf, _sz]),

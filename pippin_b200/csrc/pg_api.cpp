@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "../../include/pippin_b200.h"
+#include "../../include/pippin_b200_tools.h"
 #include "pg_kernels.h"
 #include "pg_lane.h"
 #include "pg_math.cuh"
@@ -1961,6 +1962,11 @@ int pg_phase_launch(const pg_handle* h, int phase, int* lanes_per_env, int* envs
   if (envs_per_block) *envs_per_block = c.tiles_per_block;
   if (blocks) *blocks = c.blocks;
   return PG_OK;
+}
+
+int pg_step_lanes(const pg_handle* h) {
+  if (!h) return -1;
+  return !use_lanes(h) ? 0 : h->kind == STEP_QUADS ? 4 : 1;
 }
 
 int pg_autotune(pg_handle* h, int64_t nstep) {

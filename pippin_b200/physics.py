@@ -401,6 +401,11 @@ class CudaPhysics:
             out[name] = (g.value, t.value, b.value)
         return out
 
+    def step_lanes(self) -> int:
+        """Lanes per env of the kernel step() runs in now (1 or 4: the whole
+        substep in one kernel; 0: the three phase kernels)."""
+        return self._L.pg_step_lanes(self._h)
+
     def autotune(self, nstep: int = 1):
         self._check(self._L.pg_autotune(self._h, int(nstep)))
         return self.launch()

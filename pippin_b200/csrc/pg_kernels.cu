@@ -1,4 +1,5 @@
-// Kernels of the batched FP64 physics backend.
+// Kernels of the batched FP64 physics backend: the substep of every model and
+// mode that pg_quad.cu and pg_lane.cu do not take, and the auxiliary kernels.
 //
 // A substep (crates/pippin/src/forward.rs:336-389) runs as three phase
 // kernels over the env range, each small enough for the instruction cache:

@@ -1451,6 +1451,15 @@ int pg_create(const void* blob, size_t bytes, int64_t n_envs, int device, pg_han
   if (rc) return rc;
   rc = set_const_range(h.get(), 0, n_envs);
   if (rc) return rc;
+  if (h->kind != STEP_PHASES && n_envs > 0) {
+    // a launch of no substeps: the kernel's code and its lanes' local memory
+    // are there before the first step (which must not allocate in
+    // pg_step_static)
+    StepArgs a = make_args(h.get());
+    a.count = 1;
+    LaneArgs p = lane_args(h.get(), 1);
+    CK(h->kind == STEP_QUADS ? launch_quad(a, p, h->stream) : launch_lane(a, p, h->stream));
+  }
   CK(cudaStreamSynchronize(h->stream));
   // a model compiled for PGS gets its warm-start buffers now
   if (h->dm.solver == SOLVER_PGS && (rc = pg_set_solver(h.get(), SOLVER_PGS, -1, -1.0, -1))) return rc;

@@ -69,6 +69,9 @@ MODELS = {
 }
 
 
+LANES = {"pendulum": 1, "arm3d": 1, "static_box": 0}  # the others: 4
+
+
 def _states(m, n, rng):
     q = np.tile(np.array(m.qpos0), (n, 1))
     for j in range(m.njnt):
@@ -97,6 +100,7 @@ def test_step_matches_oracle(name, n):
     m = mjcf.load_string(MODELS[name])
     blob = mjcf.to_blob(m)
     g, o = CudaPhysics(blob, n), Oracle(blob, n, threads=8)
+    assert g.step_lanes() == LANES.get(name, 4)
     o.set_solver(tolerance=1e-10, iterations=30)
     g.set_solver(tolerance=1e-10, iterations=30, warm=int(WarmStart.REF_PREV_QACC))
     rng = np.random.default_rng(n)
@@ -142,6 +146,38 @@ def test_named_shape_runs_the_phase_kernels():
         p.set(Field.QVEL, range(n), v)
         p.step(range(n), 2)
     assert _rel(a.get(Field.QACC, range(n)), b.get(Field.QACC, range(n))) < TOL
+
+
+def test_masks_that_let_pairs_touch_leave_the_one_lane_step():
+    """A model whose pairs are all masked out steps one lane an env; once
+    set_param lets geoms touch, its contacts are found like the oracle's."""
+    n = 40
+    xml = _chain(5).replace("<geom ", '<geom contype="0" conaffinity="0" ').replace('limited="true"', 'limited="false"')
+    m = mjcf.load_string(xml)
+    blob = mjcf.to_blob(m)
+    g, o = CudaPhysics(blob, n), Oracle(blob, n, threads=8)
+    for sim in (g, o):
+        sim.set_solver(tolerance=1e-10, iterations=30)
+    q, v = _states(m, n, np.random.default_rng(4))
+    g.set(Field.QPOS, range(n), q)
+    g.set(Field.QVEL, range(n), v)
+    assert g.step_lanes() == 1
+    contacts = 0
+    for t in range(6):
+        if t == 2:
+            for geom in range(len(m.geom_body)):
+                for pid in (3, 4):
+                    g.set_param(Param(pid), geom, range(n), np.ones((n, 1)))
+                    o.set_param(pid, geom, np.ones((n, 1)), 0, n)
+            assert g.step_lanes() == 0
+        for fg, fo in ((Field.QPOS, QPOS), (Field.QVEL, QVEL), (Field.QACC, QACC), (Field.CTRL, CTRL)):
+            o.set(fo, g.get(fg, range(n)))
+        g.step(range(n), 1)
+        o.step(0, n, 1)
+        assert _rel(g.get(Field.QACC, range(n)), o.get(QACC)) < TOL, t
+        np.testing.assert_array_equal(g.stats()["ncon"], o.stats()["ncon"])
+        contacts += int(g.stats()["ncon"].sum())
+    assert contacts > 0
 
 
 def test_long_calls_and_cold_start():

@@ -71,17 +71,20 @@ struct QuadLayout {
 };
 
 // x <- H^-1 x, H by rows (row i = r + 4 t on lane r, h[t][j], j <= i) and x
-// likewise: H = L' D L from the last rows on, two rows a step (D of 2 x 2
-// blocks), which halves the chain of divisions and exchanges. A step's two
-// lanes publish their rows and right-hand sides in buf. False if a pivot is
-// not positive (the same on the env's four lanes).
+// likewise: H = L' D L from the last rows on, two rows a step, which halves
+// the chain of divisions and exchanges. A step's two lanes publish their rows
+// and right-hand sides in buf; the lanes then take the later row out of the
+// earlier one, so the pivots are scalar ones (one division for both). A 2 x 2 inverse in their place is not backward stable, and H's rows
+// are nearly dependent wherever contacts are much stiffer than M: with
+// impratio 100, or solimp up to 0.9999, it cost two digits of qacc. False if a
+// pivot is not positive (the same on the env's four lanes).
 template <int N>
 __device__ __forceinline__ bool quad_factor_solve(double (&h)[(N + 3) / 4][N], double (&x)[(N + 3) / 4], double* buf, int r) {
   static_assert(N % 2 == 0, "two rows a step");
   constexpr int T = (N + 3) / 4, ROW = QuadLayout<N>::ROW;
   double *r0 = buf, *r1 = buf + ROW;
   bool ok = true;
-  double own[T], other[T];  // own row of the 2 x 2 block's inverse
+  double own[T], other[T];  // own pivot's reciprocal; the earlier row's multiple of the later
 #pragma unroll
   for (int k0 = N - 2; k0 >= 0; k0 -= 2) {
     const int k1 = k0 + 1, tk = k0 / 4;
@@ -97,14 +100,15 @@ __device__ __forceinline__ bool quad_factor_solve(double (&h)[(N + 3) / 4][N], d
       r1[N] = x[tk];
     }
     __syncwarp();
-    const double d0 = r0[k0], d1 = r1[k1], o = r1[k0], x0 = r0[N], x1 = r1[N];
-    const double det = d0 * d1 - o * o;
+    const double d1 = r1[k1], o = r1[k0], x1 = r1[N];
+    const double det = r0[k0] * d1 - o * o;
     ok = ok && d1 > 0.0 && det > 0.0;
-    const double id = 1.0 / det;
-    const double i00 = d1 * id, i11 = d0 * id, i10 = -(o * id);
+    const double inv = 1.0 / (d1 * det);  // of both pivots, d1 and det / d1
+    const double i1 = det * inv, i0 = d1 * (d1 * inv), mul = o * i1;
+    const double x0 = r0[N] - mul * x1;
     if ((r & 2) == (k0 & 2)) {
-      own[tk] = (r & 1) ? i11 : i00;
-      other[tk] = i10;
+      own[tk] = (r & 1) ? i1 : i0;
+      other[tk] = mul;
     }
     double l0[T], l1[T];
 #pragma unroll
@@ -112,16 +116,18 @@ __device__ __forceinline__ bool quad_factor_solve(double (&h)[(N + 3) / 4][N], d
       l0[t] = l1[t] = 0.0;
       if (4 * t < k0) {
         if (4 * t + 3 < k0 || 4 * t + r < k0) {
-          double a0 = r0[4 * t + r], a1 = r1[4 * t + r];
-          l0[t] = a0 * i00 + a1 * i10;
-          l1[t] = a0 * i10 + a1 * i11;
+          const double a1 = r1[4 * t + r], a0 = r0[4 * t + r] - mul * a1;
+          r0[4 * t + r] = a0;
+          l0[t] = a0 * i0;
+          l1[t] = a1 * i1;
         }
         x[t] -= l0[t] * x0 + l1[t] * x1;
       }
     }
+    __syncwarp();
 #pragma unroll
     for (int j = 0; j < k0; j++) {
-      double e0 = r0[j], e1 = r1[j];
+      const double e0 = r0[j], e1 = r1[j];
 #pragma unroll
       for (int t = 0; t < T; t++)
         if (4 * t < k0 && j <= 4 * t + 3) h[t][j] -= l0[t] * e0 + l1[t] * e1;
@@ -135,9 +141,11 @@ __device__ __forceinline__ bool quad_factor_solve(double (&h)[(N + 3) / 4][N], d
   for (int k0 = 0; k0 < N; k0 += 2) {
     const int tk = k0 / 4;
     double b = x[tk] - s[tk];
-    double y = own[tk] * b + other[tk] * __shfl_xor_sync(FULL, b, 1);
+    double y = own[tk] * (b - other[tk] * __shfl_xor_sync(FULL, b, 1));  // (the earlier row's lane)
+    const double y0 = __shfl_sync(FULL, y, k0 % 4, 4);
+    if (r & 1) y = own[tk] * (b - h[tk][k0] * y0);
     if ((r & 2) == (k0 & 2)) x[tk] = y;
-    double y0 = __shfl_sync(FULL, y, k0 % 4, 4), y1 = __shfl_sync(FULL, y, k0 % 4 + 1, 4);
+    const double y1 = __shfl_sync(FULL, y, k0 % 4 + 1, 4);
 #pragma unroll
     for (int t = tk; t < T; t++)
       if (4 * t + r > k0 + 1) s[t] += h[t][k0] * y0 + h[t][k0 + 1] * y1;

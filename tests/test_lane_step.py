@@ -197,3 +197,62 @@ def test_long_calls_and_cold_start():
         b.step(range(n), 1)
     for f in (Field.QPOS, Field.QVEL, Field.QACC):
         np.testing.assert_array_equal(a.get(f, range(n)), b.get(f, range(n)))
+
+
+# light limbs on a heavy trunk, stiff contacts and limits, tangents far softer
+# and far harder than the normals
+HARD = {
+    "light_limbs": dict(limb="2", trunk="40000"),
+    "impratio_100": dict(opt='impratio="100"'),
+    "impratio_0.01": dict(opt='impratio="0.01"'),
+    "stiff": dict(opt='o_solref="0.009 1"', solimp=(0.95, 0.9999, 0.0005, 0.5, 2.0)),
+    "light_and_stiff": dict(limb="2", trunk="40000", opt='impratio="100"', solimp=(0.95, 0.9999, 0.0005, 0.5, 2.0)),
+}
+
+
+@pytest.mark.parametrize("hard", list(HARD))
+@pytest.mark.parametrize("name", ["free_3_limbs", "free_5_limbs"])
+def test_hard_models_lose_no_more_than_in_the_phase_kernels(name, hard):
+    """M and the Newton systems with condition numbers two to six decades
+    above the other models': the four-lane step's qacc is as near to the
+    oracle's as that of the phase kernels. Both factorisations are backward
+    stable, so their errors differ by a small factor (8 is allowed, above a
+    floor of 1e-13, some rounding of a well-conditioned step)."""
+    n = 120
+    opt = HARD[hard]
+    xml = MODELS[name].replace('density="400"', f'density="{opt.get("trunk", 400)}"')
+    if "limb" in opt:
+        for geom in ('size="0.05"/>', 'size="0.07"/>', 'euler="10 20 30"/>'):
+            xml = xml.replace(geom, f'{geom[:-2]} density="{opt["limb"]}"/>')
+        xml = xml.replace('armature="0.02"', "").replace('armature="0.01"', "")
+    xml = xml.replace('iterations="30"/>', f'iterations="30" {opt.get("opt", "")}/>')
+    m = mjcf.load_string(xml)
+    m.solimp = opt.get("solimp", m.solimp)
+    blob = mjcf.to_blob(m)
+    lanes, phases, o = CudaPhysics(blob, n), CudaPhysics(blob, n), Oracle(blob, n, threads=8)
+    phases.set_launch(16, 4)
+    assert (lanes.step_lanes(), phases.step_lanes()) == (4, 0)
+    for sim in (lanes, phases, o):
+        sim.set_solver(tolerance=1e-10, iterations=60)
+    rng = np.random.default_rng(17)
+    q, v = _states(m, n, rng)
+    lanes.set(Field.QPOS, range(n), q)
+    lanes.set(Field.QVEL, range(n), v)
+    worst, rows = [0.0, 0.0], 0
+    for _ in range(6):
+        lanes.set(Field.CTRL, range(n), rng.uniform(-1, 1, (n, m.nu)))
+        for fg, fo in ((Field.QPOS, QPOS), (Field.QVEL, QVEL), (Field.QACC, QACC), (Field.CTRL, CTRL)):
+            s = lanes.get(fg, range(n))
+            o.set(fo, s)
+            phases.set(fg, range(n), s)
+        for p in (lanes, phases):
+            p.step(range(n), 1)
+        o.step(0, n, 1)
+        ref = o.get(QACC)
+        scale = np.maximum(np.abs(ref).max(axis=1), 1.0)
+        for k, p in enumerate((lanes, phases)):
+            worst[k] = max(worst[k], float((np.abs(p.get(Field.QACC, range(n)) - ref).max(axis=1) / scale).max()))
+        assert not lanes.stats()["status"].any()
+        rows += int(lanes.stats()["nrows"].sum())
+    assert rows > 0
+    assert worst[0] <= 8 * max(worst[1], 1e-13), worst

@@ -62,7 +62,8 @@ __device__ __forceinline__ void walk_body(const DModel& m, int b, const double* 
   pos = pos + mv(xm, ld3(m.body_pos + 3 * b));
   Q4 bq = ld4(m.body_quat + 4 * b);
   bool turned = false;  // mat no longer of quat
-  if (bq.w != 1.0) {
+  // (a frame turned by 2e-8 or less has w == 1 all the same)
+  if (bq.w != 1.0 || bq.x != 0.0 || bq.y != 0.0 || bq.z != 0.0) {
     quat = q_mul(quat, bq);
     turned = true;
   }

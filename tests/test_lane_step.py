@@ -256,3 +256,43 @@ def test_hard_models_lose_no_more_than_in_the_phase_kernels(name, hard):
         rows += int(lanes.stats()["nrows"].sum())
     assert rows > 0
     assert worst[0] <= 8 * max(worst[1], 1e-13), worst
+
+
+def _oracle_step(g, o, n, tol):
+    """One substep of both from g's states: the largest relative difference,
+    which must be below tol."""
+    for fg, fo in ((Field.QPOS, QPOS), (Field.QVEL, QVEL), (Field.QACC, QACC), (Field.CTRL, CTRL)):
+        if g.dims().width(fg):
+            o.set(fo, g.get(fg, range(n)))
+    g.step(range(n), 1)
+    o.step(0, n, 1)
+    sg, so = g.stats(), o.stats()
+    np.testing.assert_array_equal(sg["ncon"], so["ncon"])
+    np.testing.assert_array_equal(sg["nrows"], so["nrows"])
+    assert not sg["status"].any()
+    for fg, fo in ((Field.QACC, QACC), (Field.QVEL, QVEL), (Field.QPOS, QPOS)):
+        assert _rel(g.get(fg, range(n)), o.get(fo)) < tol, fg
+    return so
+
+
+@pytest.mark.parametrize("name", ["chain_6", "free_3_limbs", "pendulum_chain"])
+def test_body_frames_turned_by_less_than_the_real_part_shows(name):
+    """A body frame turned by 2e-8 has a quaternion whose real part rounds to
+    one; the turn still tilts all that hangs on it."""
+    n = 33
+    xml = MODELS.get(name) or _chain(4).replace("<geom ", '<geom contype="0" conaffinity="0" ').replace(
+        'limited="true"', 'limited="false"')
+    xml = xml.replace('<body pos="0.12 0 0" euler="0 0 0">', '<body pos="0.12 0 0" quat="1 9e-9 -9e-9 9e-9">')
+    xml = xml.replace('euler="0 0 0"', 'quat="1 9e-9 -9e-9 9e-9"')
+    assert "9e-9" in xml
+    m = mjcf.load_string(xml)
+    blob = mjcf.to_blob(m)
+    assert any(q[0] == 1.0 and q[1] != 0.0 for q in np.reshape(m.body_quat, (-1, 4)))
+    g, o = CudaPhysics(blob, n), Oracle(blob, n, threads=4)
+    assert g.step_lanes() == (1 if name == "pendulum_chain" else 4)
+    for sim in (g, o):
+        sim.set_solver(tolerance=1e-10, iterations=30)
+    q, v = _states(m, n, np.random.default_rng(2))
+    g.set(Field.QPOS, range(n), q)
+    g.set(Field.QVEL, range(n), v)
+    _oracle_step(g, o, n, TOL)

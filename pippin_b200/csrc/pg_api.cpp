@@ -410,13 +410,11 @@ struct Handle {
   bool mlp_loaded = false;
   std::vector<double> base_params;
   // the one- and four-lane substeps: whether the model takes one (STEP_*),
-  // whether the caller asked for a phase-kernel shape instead, and their copy
-  // of the parameter blocks ([32 envs][k][lane], made by the first
-  // pg_set_param that changes a physical parameter; until then every env
-  // reads env 0's block)
+  // whether the caller asked for a phase-kernel shape instead, and the device
+  // word that says whether pg_set_param has written a physical parameter
   int kind = STEP_PHASES;
   bool forced_shape = false;
-  double* prm_lanes = nullptr;
+  int* mixed = nullptr;
   int warm_mode = WARM_REF_PREV_QACC;
   SubstepCfg cfg{{16, 4, 0}, {32, 4, 0}, {16, 4, 0}};
   int sm_count = 0;
@@ -746,8 +744,7 @@ bool use_lanes(const Handle* h) {
 }
 LaneArgs lane_args(const Handle* h, int64_t count) {
   LaneArgs p{};
-  p.prm = h->prm_lanes ? h->prm_lanes : h->params;
-  p.uniform = h->prm_lanes ? 0 : 1;
+  p.mixed = h->mixed;
   p.sms = h->sm_count;
   // a full warp's worth of envs only once every SM sub-partition has a warp:
   // below that fewer envs a warp end the Newton loop sooner
@@ -1317,7 +1314,7 @@ void destroy(pg_handle* h) {
   cudaSetDevice(h->device);
   clear_graphs(h);
   void* ptrs[] = {h->d_model, h->qpos, h->qvel, h->ctrl, h->qacc, h->applied, h->params, h->iters, h->ncon,
-                  h->nrows, h->status, h->scratch, h->prm_lanes, h->work, h->prev_con, h->prev_ncon, h->queue, h->order, h->b_ctrl.p, h->b_qout.p, h->b_poses_g.p,
+                  h->nrows, h->status, h->scratch, h->mixed, h->work, h->prev_con, h->prev_ncon, h->queue, h->order, h->b_ctrl.p, h->b_qout.p, h->b_poses_g.p,
                   h->b_poses_c.p, h->b_dbg.p, h->b_vals.p, h->b_ids.p, h->learn.items, h->learn.feat, h->learn.force,
                   h->learn.rows, (void*)h->learn.mlp_w, (void*)h->learn.mlp_f, (void*)h->learn.mlp_err};
   for (void* p : ptrs)
@@ -1408,6 +1405,8 @@ int pg_create(const void* blob, size_t bytes, int64_t n_envs, int device, pg_han
   CK(cudaMalloc(&h->ncon, sizeof(int32_t) * n));
   CK(cudaMalloc(&h->nrows, sizeof(int32_t) * n));
   CK(cudaMalloc(&h->status, sizeof(int32_t) * n));
+  CK(cudaMalloc(&h->mixed, sizeof(int)));
+  CK(cudaMemsetAsync(h->mixed, 0, sizeof(int), h->stream));
   CK(cudaMalloc(&h->queue, sizeof(int) * QUEUE_INTS));
   CK(cudaMalloc(&h->order, sizeof(int) * std::max<int64_t>(n, 1)));
   CK(cudaMalloc(&h->work, sizeof(double) * n * h->k.stride));
@@ -1711,41 +1710,15 @@ int pg_set_param(pg_handle* h, int param, int64_t id, int64_t start, int64_t end
   // the values go to the device, where each env's parameter block takes them
   if ((rc = grow(h, h->b_vals, sizeof(double) * len))) return rc;
   const bool physical = param != PG_PARAM_GEOM_RGBA && param != PG_PARAM_QPOS0;
-  const bool first = h->kind != STEP_PHASES && physical && !h->prm_lanes;
-  std::unique_ptr<double, cudaError_t (*)(void*)> fresh(nullptr, [](void* p) { return cudaFree(p); });
-  if (first) {
-    double* p = nullptr;
-    CK(cudaMalloc(&p, sizeof(double) * ((h->n + 31) / 32 * 32) * h->dm.pstride));
-    fresh.reset(p);
-  }
   CK(cudaMemcpyAsync(h->b_vals.p, values, sizeof(double) * len, cudaMemcpyHostToDevice, h->stream));
   CK(launch_apply_param(h->dm, h->params + start * h->dm.pstride, end - start, param, id, (const double*)h->b_vals.p, w,
-                        m.nq, h->stream));
+                        m.nq, physical ? h->mixed : nullptr, h->stream));
   if (param == PG_PARAM_BODY_MASS || param == PG_PARAM_BODY_INERTIA || param == PG_PARAM_BODY_IPOS) {
     if ((rc = set_const_range(h, start, end))) return rc;
   }
   // masks may now let pairs touch: a model that took one lane for want of
   // rows leaves it
   if ((param == PG_PARAM_GEOM_CONTYPE || param == PG_PARAM_GEOM_CONAFFINITY) && h->kind == STEP_LANES) h->kind = STEP_PHASES;
-  if (h->kind != STEP_PHASES && physical) {
-    const DModel& d = h->dm;
-    auto mirror = [&](int64_t e0, int64_t e1, int off, int cnt) {
-      return launch_mirror(h->params, h->prm_lanes, d.pstride, e0, e1, off, cnt, h->stream);
-    };
-    if (first) {
-      CK(launch_mirror(h->params, fresh.get(), d.pstride, 0, h->n, 0, d.pstride, h->stream));
-      h->prm_lanes = fresh.release();
-    } else {
-      int step;
-      const int off = param_offset(d, param, id, &step);
-      CK(mirror(start, end, off, param == PG_PARAM_BODY_INERTIA ? 9 : w));
-      if (param == PG_PARAM_BODY_MASS) CK(mirror(start, end, d.p_inertia + 9 * (int)id, 9));
-      if (param == PG_PARAM_BODY_MASS || param == PG_PARAM_BODY_INERTIA || param == PG_PARAM_BODY_IPOS) {
-        CK(mirror(start, end, d.p_body_invw, 2 * m.nbody));
-        CK(mirror(start, end, d.p_dof_invw, m.nv));
-      }
-    }
-  }
   CK(cudaStreamSynchronize(h->stream));
   return PG_OK;
 }

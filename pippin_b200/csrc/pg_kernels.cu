@@ -719,15 +719,16 @@ cudaError_t launch_substep(const StepArgs& a0, const SubstepCfg& c, cudaStream_t
 }
 
 __global__ void apply_param_kernel(const __grid_constant__ DModel d, double* params, int64_t count, int p, int64_t id,
-                                   const double* v, int w, int nq) {
+                                   const double* v, int w, int nq, int* mixed) {
   int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (mixed && e == 0) *mixed = 1;
   if (e < count) apply_param(d, params + e * d.pstride, p, id, v + e * w, nq);
 }
 
 cudaError_t launch_apply_param(const DModel& d, double* params, int64_t count, int p, int64_t id, const double* v, int w,
-                               int nq, cudaStream_t s) {
+                               int nq, int* mixed, cudaStream_t s) {
   if (count <= 0) return cudaSuccess;
-  apply_param_kernel<<<(unsigned)((count + 127) / 128), 128, 0, s>>>(d, params, count, p, id, v, w, nq);
+  apply_param_kernel<<<(unsigned)((count + 127) / 128), 128, 0, s>>>(d, params, count, p, id, v, w, nq, mixed);
   return cudaGetLastError();
 }
 

@@ -67,8 +67,7 @@ __global__ void __launch_bounds__(32) lane_kernel(const __grid_constant__ StepAr
   const bool alive = lane < L;
   const int64_t item = item0 + (alive ? lane : L - 1);  // the others repeat the last env and write nothing
   const int64_t env = A.start + item;
-  const double* pp = P.uniform ? P.prm : P.prm + (env >> 5) * (int64_t)m.pstride * 32 + (env & 31);
-  const int ps = P.uniform ? 1 : 32;
+  const double* pp = A.st.params + (*P.mixed ? env * m.pstride : 0);
   const double h = m.timestep;
 
   double q[LANE_NQ], v[N], f[N], qacc[N], hd[N];
@@ -82,7 +81,7 @@ __global__ void __launch_bounds__(32) lane_kernel(const __grid_constant__ StepAr
     const bool in = k < nv;
     v[k] = in ? A.st.qvel[env * nv + k] : 0.0;
     qacc[k] = in ? A.st.qacc[env * nv + k] : 0.0;
-    hd[k] = in ? pp[(m.p_damping + k) * ps] : 0.0;
+    hd[k] = in ? pp[m.p_damping + k] : 0.0;
     damped |= hd[k] != 0.0;
   }
   int status_all = P.sidx == 0 ? 0 : A.st.status[env];
@@ -181,7 +180,7 @@ __global__ void __launch_bounds__(32) lane_kernel(const __grid_constant__ StepAr
         }
         top++;
         path[top] = b;
-        walk_body(m, b, q, v, cdof, pp, ps, s);
+        walk_body(m, b, q, v, cdof, pp, s);
       }
     }
     // ------------------------------------------------ passive and actuator forces
@@ -206,8 +205,8 @@ __global__ void __launch_bounds__(32) lane_kernel(const __grid_constant__ StepAr
       double c = A.ctrl_seq ? A.ctrl_seq[((size_t)item * A.nstep + sidx) * nu + u] : A.st.ctrl[env * nu + u];
       if (A.ctrl_seq && alive) A.st.ctrl[env * nu + u] = c;  // rollout leaves the last controls in place
       if (m.act_ctrllimited[u]) c = clampd(c, m.act_ctrlrange[2 * u], m.act_ctrlrange[2 * u + 1]);
-      double fu = pp[(m.p_gain + u) * ps] * c + pp[(m.p_bias + 3 * u) * ps] + pp[(m.p_bias + 3 * u + 1) * ps] * (gear * ls) +
-                  pp[(m.p_bias + 3 * u + 2) * ps] * (gear * vs);
+      double fu = pp[m.p_gain + u] * c + pp[m.p_bias + 3 * u] + pp[m.p_bias + 3 * u + 1] * (gear * ls) +
+                  pp[m.p_bias + 3 * u + 2] * (gear * vs);
       if (m.act_forcelimited[u]) fu = clampd(fu, m.act_forcerange[2 * u], m.act_forcerange[2 * u + 1]);
       for (int k = a0; k < a0 + an; k++) f[m.jnt_dofadr[m.moment_jnt[k]]] += gear * m.moment_coef[k] * fu;
     }
@@ -290,15 +289,6 @@ __global__ void __launch_bounds__(32) lane_kernel(const __grid_constant__ StepAr
   }
 }
 
-__global__ void mirror_kernel(const double* params, double* lanes, int pstride, int64_t start, int64_t end, int off,
-                              int len) {
-  // a warp writes one field of 32 envs
-  int64_t e = (start & ~31ll) + (int64_t)blockIdx.x * 32 + threadIdx.x;
-  if (e < start || e >= end) return;
-  for (int k = off + threadIdx.y; k < off + len; k += blockDim.y)
-    lanes[(e >> 5) * (int64_t)pstride * 32 + (int64_t)k * 32 + (e & 31)] = params[e * pstride + k];
-}
-
 }  // namespace
 
 cudaError_t launch_lane(const StepArgs& a, const LaneArgs& p, cudaStream_t s) {
@@ -307,14 +297,6 @@ cudaError_t launch_lane(const StepArgs& a, const LaneArgs& p, cudaStream_t s) {
   if (a.m.nv <= 4) lane_kernel<4><<<(unsigned)warps, 32, 0, s>>>(a, p);
   else if (a.m.nv <= 8) lane_kernel<8><<<(unsigned)warps, 32, 0, s>>>(a, p);
   else lane_kernel<16><<<(unsigned)warps, 32, 0, s>>>(a, p);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_mirror(const double* params, double* lanes, int pstride, int64_t start, int64_t end, int off, int len,
-                          cudaStream_t s) {
-  if (end <= start || len <= 0) return cudaSuccess;
-  int64_t blocks = (end - (start & ~31ll) + 31) / 32;
-  mirror_kernel<<<(unsigned)blocks, dim3(32, 8), 0, s>>>(params, lanes, pstride, start, end, off, len);
   return cudaGetLastError();
 }
 

@@ -51,9 +51,9 @@ __device__ __forceinline__ void walk_world(const DModel& m, Walk& s) {
 }
 // forward.rs:14-90, 115-164 for body b: on entry s holds its parent's pose,
 // velocity and acceleration, on return its own; its dofs' axes go to cdof.
-// q, v: the env's state; pp / ps: its parameter block and the block's stride.
+// q, v: the env's state; pp: its parameter block.
 __device__ __forceinline__ void walk_body(const DModel& m, int b, const double* q, const double* v, double* cdof,
-                                          const double* pp, int ps, Walk& s) {
+                                          const double* pp, Walk& s) {
   V3& pos = s.pos;
   Q4& quat = s.quat;
   Sp &vel = s.vel, &acc = s.acc;
@@ -118,11 +118,11 @@ __device__ __forceinline__ void walk_body(const DModel& m, int b, const double* 
     quat = unit(quat);
     xm = q_mat(quat);
   }
-  V3 ip{pp[(m.p_ipos + 3 * b) * ps], pp[(m.p_ipos + 3 * b + 1) * ps], pp[(m.p_ipos + 3 * b + 2) * ps]};
+  V3 ip{pp[m.p_ipos + 3 * b], pp[m.p_ipos + 3 * b + 1], pp[m.p_ipos + 3 * b + 2]};
   M3 in;
 #pragma unroll
-  for (int t = 0; t < 9; t++) in.m[t] = pp[(m.p_inertia + 9 * b + t) * ps];
-  double mass = pp[(m.p_mass + b) * ps];
+  for (int t = 0; t < 9; t++) in.m[t] = pp[m.p_inertia + 9 * b + t];
+  double mass = pp[m.p_mass + b];
   // R I R' + m (|c|^2 1 - c c'), upper triangle
   V3 c = pos + mv(xm, ip);
   M3 ri = mm(xm, in);
@@ -162,12 +162,12 @@ __device__ __forceinline__ void walk_body(const DModel& m, int b, const double* 
 }
 
 // A geom's pose on its body and the half box around it (forward.rs:84-89, 217-232; primitives only).
-__device__ __forceinline__ void geom_box(const DModel& m, int g, const Walk& s, const double* pp, int ps, V3* x, M3* gm,
+__device__ __forceinline__ void geom_box(const DModel& m, int g, const Walk& s, const double* pp, V3* x, M3* gm,
                                          V3* half) {
   *x = s.pos + mv(s.mat, ld3(m.geom_pos + 3 * g));
   *gm = mm(s.mat, q_mat(ld4(m.geom_quat + 4 * g)));
   int gt = m.geom_type[g];
-  V3 z{pp[(m.p_size + 3 * g) * ps], pp[(m.p_size + 3 * g + 1) * ps], pp[(m.p_size + 3 * g + 2) * ps]};
+  V3 z{pp[m.p_size + 3 * g], pp[m.p_size + 3 * g + 1], pp[m.p_size + 3 * g + 2]};
   V3 hb = z;
   if (gt == GEOM_SPHERE) hb = V3{z.x, z.x, z.x};
   if (gt == GEOM_CAPSULE) hb = V3{z.x, z.x, z.x + z.y};

@@ -22,8 +22,11 @@ enum { LC_POS = 0, LC_N = 3, LC_T = 6, LC_MU = 9, LC_D = 10, LC_OFF = 11, LC_MAS
        LC_STRIDE = 21 };
 
 struct LaneArgs {
-  const double* prm;   // parameter blocks: see below
-  int uniform;         // 1: every env reads the block at prm; 0: blocks of 32 envs, [k][32], from env 0
+  // on the device: 0 while the envs' physical parameters are all env 0's,
+  // whose block every env then reads (one address for the whole warp); 1 once
+  // pg_set_param has written one. Read when the kernel runs, so that a
+  // captured step replays with the parameters of that time.
+  const int* mixed;
   int lanes;           // envs a warp takes (1..32)
   int sms;             // SMs of the GPU
   int sidx, nsub;      // substeps [sidx, sidx + nsub) of the call
@@ -33,9 +36,5 @@ struct LaneArgs {
 cudaError_t launch_lane(const StepArgs& a, const LaneArgs& p, cudaStream_t s);
 // The same with four lanes per env (a.m.limb_n >= 0; p.lanes at most 8).
 cudaError_t launch_quad(const StepArgs& a, const LaneArgs& p, cudaStream_t s);
-// rows [off, off + len) of the parameter blocks of envs [start, end) into the
-// lane kernel's layout
-cudaError_t launch_mirror(const double* params, double* lanes, int pstride, int64_t start, int64_t end, int off, int len,
-                          cudaStream_t s);
 
 }  // namespace pg

@@ -199,8 +199,7 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
   const int es = slot < L ? slot : L - 1;
   const int64_t item = item0 + es;
   const int64_t env = A.start + item;
-  const double* pp = P.uniform ? P.prm : P.prm + (env >> 5) * (int64_t)m.pstride * 32 + (env & 31);
-  const int ps = P.uniform ? 1 : 32;
+  const double* pp = A.st.params + (*P.mixed ? env * m.pstride : 0);
   double* ws = smem + (size_t)(threadIdx.x >> 2) * Q::stride(m.ngeom, nq);
   double *v = ws + Q::V, *cdof = ws + Q::C, *buf = ws + Q::B, *fs = buf, *xs = buf, *U = ws + Q::U, *Ms = ws + Q::M,
          *box = Ms, *q = Ms + Q::region(m.ngeom);
@@ -223,7 +222,7 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
   for (int t = 0; t < T; t++) {
     int k = r + 4 * t;
     bool in = k < nv;
-    hd[t] = in ? pp[(m.p_damping + k) * ps] : 0.0;
+    hd[t] = in ? pp[m.p_damping + k] : 0.0;
     qw[t] = in ? A.st.qacc[env * nv + k] : 0.0;
     chain[t] = in ? (unsigned)m.body_dofmask[m.dof_body[k]] & ((2u << k) - 1u) : 0u;
     damped |= hd[t] != 0.0;
@@ -247,7 +246,7 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
           for (int g = m.body_gadr[b] + g0; g < m.body_gadr[b + 1]; g += step) {
             V3 x, half;
             M3 gm;
-            geom_box(m, g, s, pp, ps, &x, &gm, &half);
+            geom_box(m, g, s, pp, &x, &gm, &half);
             st3(box + 6 * g, x);
             st3(box + 6 * g + 3, half);
             if (alive)
@@ -312,7 +311,7 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
           if (l0 == 0 && k == 0 && m.limb_n > 4) end = s;
           if (k < 0 || a0 + k < a1) {
             int b = k < 0 ? m.trunk[m.trunk_n + k] : m.limb_body[a0 + k];
-            walk_body(m, b, q, v, cdof, pp, ps, s);
+            walk_body(m, b, q, v, cdof, pp, s);
             if (k < 0) geoms(b, r, 4, s);
             else geoms(b, 0, 1, s);
             keep(k < 0 ? tr + 16 * (m.trunk_n + k) : lb + 16 * k, s.I, s.fr);
@@ -393,8 +392,8 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
         hits.n = 0;
         int nh = 0;
         if (keep) {
-          unsigned t1 = (unsigned)pp[(m.p_contype + g1) * ps], a1 = (unsigned)pp[(m.p_conaff + g1) * ps];
-          unsigned t2 = (unsigned)pp[(m.p_contype + g2) * ps], a2 = (unsigned)pp[(m.p_conaff + g2) * ps];
+          unsigned t1 = (unsigned)pp[m.p_contype + g1], a1 = (unsigned)pp[m.p_conaff + g1];
+          unsigned t2 = (unsigned)pp[m.p_contype + g2], a2 = (unsigned)pp[m.p_conaff + g2];
           keep = (t1 & a2) != 0 || (t2 & a1) != 0;
         }
         if (keep) {
@@ -404,12 +403,12 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
             const double* pm = gmat + (size_t)9 * gpl * L;
             V3 pn{pm[2 * L], pm[5 * L], pm[8 * L]};
             V3 pc = ld3(box + 6 * gpl), x = ld3(box + 6 * go);
-            double rad = pp[(m.p_size + 3 * go) * ps];
+            double rad = pp[m.p_size + 3 * go];
             V3 ax{0, 0, 0}, e{0, 0, 0};
             if (to == GEOM_CAPSULE) {
               const double* gm = gmat + (size_t)9 * go * L;
               ax = V3{gm[2 * L], gm[5 * L], gm[8 * L]};
-              e = ax * pp[(m.p_size + 3 * go + 1) * ps];
+              e = ax * pp[m.p_size + 3 * go + 1];
             }
             V3 nn = gpl == g1 ? pn : -pn;
             for (int k = 0; k < (to == GEOM_CAPSULE ? 2 : 1); k++) {
@@ -424,7 +423,7 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
 #pragma unroll
               for (int t = 0; t < 9; t++) gm.m[t] = gmat[(size_t)(9 * g + t) * L];
               return GPose{ty, ld3(box + 6 * g), gm,
-                           V3{pp[(m.p_size + 3 * g) * ps], pp[(m.p_size + 3 * g + 1) * ps], pp[(m.p_size + 3 * g + 2) * ps]}, 0};
+                           V3{pp[m.p_size + 3 * g], pp[m.p_size + 3 * g + 1], pp[m.p_size + 3 * g + 2]}, 0};
             };
             collide_primitive(pose(g1, ty1), pose(g2, ty2), m.margin, hits);
             nh = hits.n < MAX_HITS ? hits.n : MAX_HITS;
@@ -442,8 +441,8 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
         if (nh > 0) {
           int b1 = m.geom_body[g1], b2 = m.geom_body[g2];
           unsigned k1 = (unsigned)m.body_dofmask[b1], k2 = (unsigned)m.body_dofmask[b2];
-          double mu = fmax(pp[(m.p_friction + g1) * ps], pp[(m.p_friction + g2) * ps]);
-          double tran = pp[(m.p_body_invw + 2 * b1) * ps] + pp[(m.p_body_invw + 2 * b2) * ps];
+          double mu = fmax(pp[m.p_friction + g1], pp[m.p_friction + g2]);
+          double tran = pp[m.p_body_invw + 2 * b1] + pp[m.p_body_invw + 2 * b2];
           double dpyr = 2.0 * mu * mu * (1.0 + mu * mu) * tran / m.impratio;
 #pragma unroll 1
           for (int k = 0; k < nh; k++) {
@@ -500,8 +499,8 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
       double c = A.ctrl_seq ? A.ctrl_seq[((size_t)item * A.nstep + sidx) * nu + u] : A.st.ctrl[env * nu + u];
       if (A.ctrl_seq && alive) A.st.ctrl[env * nu + u] = c;  // rollout leaves the last controls in place
       if (m.act_ctrllimited[u]) c = clampd(c, m.act_ctrlrange[2 * u], m.act_ctrlrange[2 * u + 1]);
-      double fu = pp[(m.p_gain + u) * ps] * c + pp[(m.p_bias + 3 * u) * ps] + pp[(m.p_bias + 3 * u + 1) * ps] * (gear * ls) +
-                  pp[(m.p_bias + 3 * u + 2) * ps] * (gear * vs);
+      double fu = pp[m.p_gain + u] * c + pp[m.p_bias + 3 * u] + pp[m.p_bias + 3 * u + 1] * (gear * ls) +
+                  pp[m.p_bias + 3 * u + 2] * (gear * vs);
       if (m.act_forcelimited[u]) fu = clampd(fu, m.act_forcerange[2 * u], m.act_forcerange[2 * u + 1]);
       U[u] = fu;
     }
@@ -702,7 +701,7 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
             if (lo < 0.0 || hi < 0.0) {
               double sg = lo < 0.0 ? 1.0 : -1.0, sep = lo < 0.0 ? lo : hi;
               double imp = row_impedance(m.solimp, sep);
-              double D = sg / fmax((1.0 - imp) / imp * pp[(m.p_dof_invw + k) * ps], 1e-15);
+              double D = sg / fmax((1.0 - imp) / imp * pp[m.p_dof_invw + k], 1e-15);
               double e = rb * (sg * v[k]) + rk * imp * sep;  // -aref
 #pragma unroll
               for (int t = 0; t < T; t++)

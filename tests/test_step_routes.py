@@ -1,0 +1,103 @@
+"""What must hold whichever kernel a step runs in: a captured step replays with
+the parameters of the time it is replayed at, and setting parameters costs no
+device memory.
+
+Two handles start from the same states; one replays a captured step, the other
+steps live after the same calls. They may run different kernels, so they agree
+within the per-step bar of the other parity tests, 1e-10.
+"""
+import numpy as np
+import pytest
+import torch
+
+from pippin_b200 import CudaPhysics, Field, Param, _native, mjcf, scenes
+from tests.test_lane_step import MODELS, TOL, _rel, _states
+
+pytestmark = pytest.mark.gpu
+
+
+class Capture:
+    """What runs inside, recorded from the handle's stream."""
+
+    def __init__(self, phys):
+        self.stream = torch.cuda.ExternalStream(phys.stream())
+        self.graph = torch.cuda.CUDAGraph()
+
+    def __enter__(self):
+        torch.cuda.synchronize()
+        self.scope = torch.cuda.stream(self.stream)
+        self.scope.__enter__()
+        self.graph.capture_begin(capture_error_mode="thread_local")
+        return self
+
+    def __exit__(self, *exc):
+        self.graph.capture_end()
+        self.scope.__exit__(None, None, None)
+
+    def replay(self):
+        with torch.cuda.stream(self.stream):
+            self.graph.replay()
+
+
+def _pair(xml, n, seed):
+    m = mjcf.load_string(xml)
+    blob = mjcf.to_blob(m)
+    a, b = CudaPhysics(blob, n), CudaPhysics(blob, n)
+    q, v = _states(m, n, np.random.default_rng(seed))
+
+    def start():
+        for p in (a, b):
+            p.set(Field.QPOS, range(n), q)
+            p.set(Field.QVEL, range(n), v)
+            p.set(Field.QACC, range(n), np.zeros((n, m.nv)))
+
+    start()
+    return m, a, b, start
+
+
+def _static(p, n, nstep=1):
+    assert _native.load().pg_step_static(p._h, 0, n, nstep) == 0, _native.last_error()
+
+
+@pytest.mark.parametrize("name", ["ant", "pendulum", "chain_6", "static_box"])
+def test_a_captured_step_takes_the_parameters_of_its_replay(name):
+    n = 24
+    m, a, b, start = _pair(MODELS[name], n, 21)
+    for p in (a, b):
+        _static(p, n)  # loads the library's device image
+        p.synchronize()
+    with Capture(a) as c:
+        _static(a, n, 2)
+    rng = np.random.default_rng(22)
+    start()
+    base = CudaPhysics(mjcf.to_blob(m), n)
+    for f in (Field.QPOS, Field.QVEL):
+        base.set(f, range(n), a.get(f, range(n)))
+    body = m.nbody - 1
+    mass = np.asarray(m.body_mass[body]) * rng.uniform(0.5, 2.0, (n, 1))
+    damp = rng.uniform(0.1, 2.0, (n, 1))
+    fric = rng.uniform(0.2, 1.5, (n, 1))
+    for p in (a, b):
+        for pid, elem, val in ((5, body, mass), (6, m.nv - 1, damp), (0, 0, fric)):
+            p.set_param(Param(pid), elem, range(n), val)
+    c.replay()
+    a.synchronize()  # (the static scratch is shared: one handle at a time)
+    for p in (b, base):
+        _static(p, n, 2)
+        p.synchronize()
+    for f in (Field.QACC, Field.QVEL, Field.QPOS):
+        assert _rel(a.get(f, range(n)), b.get(f, range(n))) < TOL, f
+    assert _rel(a.get(Field.QACC, range(n)), base.get(Field.QACC, range(n))) > 1e-3  # the parameters matter
+
+
+@pytest.mark.parametrize("solver", [0, 1], ids=["newton", "pgs"])
+def test_set_param_takes_no_device_memory(solver):
+    """(But for the values themselves: a copy of the parameter blocks of these
+    envs would take 56 MB.)"""
+    free = 0
+    for n in (4, 16384):  # the small handle loads the kernels
+        p = CudaPhysics(scenes.ant_xml(), n)
+        p.set_solver(kind=solver)
+        free = torch.cuda.mem_get_info()[0]
+        p.set_param(Param.BODY_MASS, 1, range(n), np.full((n, 1), 2.0))
+    assert free - torch.cuda.mem_get_info()[0] < 8 << 20

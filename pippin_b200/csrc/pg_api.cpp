@@ -742,6 +742,11 @@ int set_const_range(Handle* h, int64_t start, int64_t end) {
 bool use_lanes(const Handle* h) {
   return h->kind != STEP_PHASES && !h->forced_shape && h->dm.solver == SOLVER_NEWTON && h->warm_mode != WARM_LEARNED;
 }
+// Whether the caller is capturing the handle's stream.
+bool capturing(const Handle* h) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(h->stream, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+}
 LaneArgs lane_args(const Handle* h, int64_t count) {
   LaneArgs p{};
   p.mixed = h->mixed;
@@ -1358,9 +1363,11 @@ int internal_step_args(pg_handle* h, int64_t start, int64_t end, int64_t nstep, 
   *device = h->device;
   return PG_OK;
 }
-// The same step one lane per env, where the handle's substeps run so.
+// The same step on one or four lanes an env, where the handle's substeps run
+// so. Not into a capture where the choice of one lane rests on the masks:
+// pg_set_param may let the pairs touch before a replay.
 bool internal_step_lanes(pg_handle* h, const StepArgs& a, int64_t start, int64_t end, int64_t nstep, int* rc) {
-  if (!use_lanes(h)) return false;
+  if (!use_lanes(h) || (h->kind == STEP_LANES && !h->hm.pairs.empty() && capturing(h))) return false;
   *rc = enqueue_lanes(h, a, start, end, nstep);
   return true;
 }

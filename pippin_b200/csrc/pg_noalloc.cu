@@ -90,7 +90,7 @@ extern "C" int pg_step_static(pg_handle* h, int64_t start, int64_t end, int64_t 
   int rc = pg::internal_step_args(h, start, end, nstep, &a, &cfg, &stream, &device);
   if (rc != PG_OK) return rc;
   if (end == start || nstep == 0) return PG_OK;
-  // one lane per env needs no tile scratch at all
+  // one or four lanes an env need no tile scratch at all
   if (pg::internal_step_lanes(h, a, start, end, nstep, &rc)) return rc;
   unsigned char* base = nullptr;  // internal_step_args made the handle's device current
   if ((rc = scratch_address(&base)) != PG_OK) return rc;

@@ -11,7 +11,7 @@ import pytest
 import torch
 
 from pippin_b200 import CudaPhysics, Field, Param, _native, mjcf, scenes
-from tests.test_lane_step import MODELS, TOL, _rel, _states
+from tests.test_lane_step import MODELS, TOL, _chain, _rel, _states
 
 pytestmark = pytest.mark.gpu
 
@@ -101,3 +101,27 @@ def test_set_param_takes_no_device_memory(solver):
         free = torch.cuda.mem_get_info()[0]
         p.set_param(Param.BODY_MASS, 1, range(n), np.full((n, 1), 2.0))
     assert free - torch.cuda.mem_get_info()[0] < 8 << 20
+
+
+def test_a_captured_step_finds_the_contacts_that_new_masks_allow():
+    n = 40
+    xml = _chain(5).replace("<geom ", '<geom contype="0" conaffinity="0" ').replace('limited="true"', 'limited="false"')
+    m, a, b, start = _pair(xml, n, 4)
+    assert a.step_lanes() == 1
+    for p in (a, b):
+        _static(p, n)
+        p.synchronize()
+    with Capture(a) as c:
+        _static(a, n)
+    start()
+    for p in (a, b):
+        for geom in range(len(m.geom_body)):
+            for pid in (3, 4):
+                p.set_param(Param(pid), geom, range(n), np.ones((n, 1)))
+    c.replay()
+    a.synchronize()
+    _static(b, n)
+    b.synchronize()
+    assert b.stats()["ncon"].sum() > 0
+    np.testing.assert_array_equal(a.stats()["ncon"], b.stats()["ncon"])
+    assert _rel(a.get(Field.QACC, range(n)), b.get(Field.QACC, range(n))) < TOL

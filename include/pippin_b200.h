@@ -144,7 +144,8 @@ int pg_step_device(pg_handle* h, int64_t start, int64_t end, int64_t nstep, cons
  * PG_ERR_UNSUPPORTED. Every call looks the array's device address up again
  * (so a context the host program resets and makes again is followed); the
  * first call on a device also loads the library's device image there, so make
- * it before any stream capture. A captured call keeps the solver
+ * it before any stream capture (pg_step and pg_step_device refuse to be
+ * captured: they replay graphs of their own). A captured call keeps the solver
  * settings of its capture and reads the parameters of its replay. All calls share the array and keep its last
  * contents: calls that overlap on the GPU race. Stream-ordered like pg_step. */
 int pg_step_static(pg_handle* h, int64_t start, int64_t end, int64_t nstep);

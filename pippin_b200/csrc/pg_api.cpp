@@ -747,6 +747,9 @@ bool capturing(const Handle* h) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(h->stream, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
 }
+int refuse_capture() {
+  return fail(PG_ERR_CUDA, "the handle's stream is being captured (pg_step replays graphs of its own; pg_step_static can be captured)");
+}
 LaneArgs lane_args(const Handle* h, int64_t count) {
   LaneArgs p{};
   p.mixed = h->mixed;
@@ -1500,6 +1503,7 @@ int pg_step(pg_handle* h, int64_t start, int64_t end, int64_t nstep) {
   if (nstep < 0 || nstep > (1 << 30)) return fail(PG_ERR_INVALID, "nstep out of range");
   if (end == start || nstep == 0) return PG_OK;
   CK(cudaSetDevice(h->device));
+  if (capturing(h)) return refuse_capture();
   if (use_lanes(h)) return enqueue_lanes(h, make_args(h), start, end, nstep);
   if (h->graph_version != h->version) {
     clear_graphs(h);
@@ -1549,6 +1553,7 @@ int pg_step_device(pg_handle* h, int64_t start, int64_t end, int64_t nstep, cons
   if (end > start && h->hm.nu > 0) {
     if (!ctrl_dev) return fail(PG_ERR_INVALID, "ctrl_dev is NULL");
     CK(cudaSetDevice(h->device));
+    if (nstep > 0 && capturing(h)) return refuse_capture();  // before the controls are recorded
     CK(cudaMemcpyAsync(h->ctrl + start * h->hm.nu, ctrl_dev, sizeof(double) * (end - start) * h->hm.nu,
                        cudaMemcpyDeviceToDevice, h->stream));
   }

@@ -1,6 +1,6 @@
 """What must hold whichever kernel a step runs in: a captured step replays with
-the parameters of the time it is replayed at, and setting parameters costs no
-device memory.
+the parameters of the time it is replayed at, calls that a caller's stream
+capture cannot take are refused, and setting parameters costs no device memory.
 
 Two handles start from the same states; one replays a captured step, the other
 steps live after the same calls. They may run different kernels, so they agree
@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 import torch
 
-from pippin_b200 import CudaPhysics, Field, Param, _native, mjcf, scenes
+from pippin_b200 import CudaPhysics, Field, Param, PhysicsError, _native, mjcf, scenes
 from tests.test_lane_step import MODELS, TOL, _chain, _rel, _states
 
 pytestmark = pytest.mark.gpu
@@ -125,3 +125,22 @@ def test_a_captured_step_finds_the_contacts_that_new_masks_allow():
     assert b.stats()["ncon"].sum() > 0
     np.testing.assert_array_equal(a.stats()["ncon"], b.stats()["ncon"])
     assert _rel(a.get(Field.QACC, range(n)), b.get(Field.QACC, range(n))) < TOL
+
+
+@pytest.mark.parametrize("name", ["ant", "pendulum", "static_box"])
+def test_steps_that_cannot_be_captured_are_refused(name):
+    """pg_step and pg_step_device replay graphs of their own: under a caller's
+    capture they return an error, whichever kernel the handle steps in, and
+    the handle steps on afterwards."""
+    n = 8
+    m, a, b, _ = _pair(MODELS[name], n, 5)
+    ctrl = torch.zeros(n, max(m.nu, 1), dtype=torch.float64, device="cuda")
+    with Capture(a):
+        with pytest.raises(PhysicsError, match="captur"):
+            a.step(range(n), 1)
+        with pytest.raises(PhysicsError, match="captur"):
+            a.step_device(range(n), 1, ctrl.data_ptr())
+    for p in (a, b):
+        p.step(range(n), 1)
+        p.synchronize()
+    np.testing.assert_array_equal(a.get(Field.QACC, range(n)), b.get(Field.QACC, range(n)))

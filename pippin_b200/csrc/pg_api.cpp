@@ -389,6 +389,7 @@ struct DevArena {
 struct Handle {
   HostModel hm;
   DModel dm{};
+  LaneModel lm{};
   WsLayout w{}, wn{};
   ScrLayout s{};
   WorkLayout k{};
@@ -624,7 +625,7 @@ std::vector<int> dmodel_pointer_fields() {
 #define PF(f) o.push_back((int)offsetof(DModel, f))
   PF(body_parent); PF(body_jntadr); PF(body_jntnum); PF(body_dofadr); PF(body_dofnum); PF(body_lastdof);
   PF(body_dofmask); PF(body_pos); PF(body_quat); PF(level_adr); PF(level_body); PF(child_adr); PF(child_list);
-  PF(jnt_type); PF(jnt_qposadr); PF(jnt_dofadr); PF(jnt_limited); PF(jnt_pos); PF(jnt_axis); PF(jnt_unit); PF(jnt_range);
+  PF(jnt_type); PF(jnt_qposadr); PF(jnt_dofadr); PF(jnt_limited); PF(jnt_pos); PF(jnt_axis); PF(jnt_range);
   PF(jnt_stiffness); PF(jnt_springref); PF(dof_body); PF(dof_parent); PF(dof_armature); PF(dof_block);
   PF(block_adr); PF(dofact_adr); PF(dofact_u); PF(dofact_coef); PF(geom_type); PF(geom_body); PF(geom_dataid);
   PF(geom_pos); PF(geom_quat); PF(pair_g); PF(cam_body); PF(cam_pos); PF(cam_quat); PF(act_gear);
@@ -633,7 +634,6 @@ std::vector<int> dmodel_pointer_fields() {
   PF(eq_solimp); PF(qpos0); PF(hull_vadr); PF(hull_vnum); PF(hull_vert); PF(hull_fadr); PF(hull_fnum);
   PF(hull_face); PF(hull_fvadr); PF(hull_fvnum); PF(hull_fv); PF(hull_eadr); PF(hull_enum); PF(hull_edge);
   PF(hull_eface); PF(hull_nbadr); PF(hull_nbnum); PF(hull_nb); PF(hull_seed);
-  PF(trunk); PF(limb_adr); PF(limb_body); PF(body_gadr); PF(pair_pack); PF(dof_limq); PF(dof_range);
 #undef PF
   return o;
 }
@@ -752,6 +752,7 @@ int refuse_capture() {
 }
 LaneArgs lane_args(const Handle* h, int64_t count) {
   LaneArgs p{};
+  p.t = h->lm;
   p.mixed = h->mixed;
   p.sms = h->sm_count;
   // a full warp's worth of envs only once every SM sub-partition has a warp:
@@ -923,7 +924,7 @@ bool pair_masked(const HostModel& m, size_t p) {
 // The substep a model's Newton steps take (STEP_*): see the rule's figures at
 // the definition of use_lanes. Both kernels hold one tree of at most 16 dofs
 // and need the bodies depth first and explicit damping.
-int step_kind(const HostModel& m, const DModel& d) {
+int step_kind(const HostModel& m, const LaneModel& t) {
   if (m.nv < 1 || m.nv > LANE_NV || m.nq > LANE_NQ || m.dof_blocks.size() != 2 || m.neq > 0 || m.integrator != 0)
     return STEP_PHASES;
   std::vector<int> path = {0};
@@ -935,10 +936,10 @@ int step_kind(const HostModel& m, const DModel& d) {
   bool rows = false;
   for (int j = 0; j < m.njnt; j++) rows |= m.jnt_limited[j] && (m.jnt_type[j] == JNT_HINGE || m.jnt_type[j] == JNT_SLIDE);
   for (size_t p = 0; 2 * p + 1 < m.pairs.size(); p++) rows |= !pair_masked(m, p);
-  if (!rows && d.limb_n < 3) return STEP_LANES;
+  if (!rows && t.limb_n < 3) return STEP_LANES;
   // four lanes: limbs that are chains, primitive pairs, at most one violated
   // side a limit, geoms in body order
-  if (d.limb_n < 0 || d.trunk_n > LANE_DEPTH || d.limb_max > LANE_DEPTH || m.nu > QUAD_NU || m.ngeom > LANE_GEOM)
+  if (t.limb_n < 0 || t.trunk_n > LANE_DEPTH || t.limb_max > LANE_DEPTH || m.nu > QUAD_NU || m.ngeom > LANE_GEOM)
     return STEP_PHASES;
   for (int g = 1; g < m.ngeom; g++)
     if (m.geom_body[g] < m.geom_body[g - 1]) return STEP_PHASES;
@@ -1020,10 +1021,10 @@ int build_device_model(Handle* h) {
     chains = chains && nchild(b) == 0;
     limb_adr.push_back((int)limb_body.size());
   }
-  d.trunk_n = (int)trunk.size();
-  d.limb_n = chains ? (int)limb_adr.size() - 1 : -1;
-  d.limb_max = 0;
-  for (int l = 0; l < d.limb_n; l++) d.limb_max = std::max(d.limb_max, limb_adr[l + 1] - limb_adr[l]);
+  h->lm.trunk_n = (int)trunk.size();
+  h->lm.limb_n = chains ? (int)limb_adr.size() - 1 : -1;
+  h->lm.limb_max = 0;
+  for (int l = 0; l < h->lm.limb_n; l++) h->lm.limb_max = std::max(h->lm.limb_max, limb_adr[l + 1] - limb_adr[l]);
   for (int b = 0; b <= nb; b++)
     while (body_gadr[b] < m.ngeom && m.geom_body[body_gadr[b]] < b) body_gadr[b]++;
   std::vector<int> dof_limq(std::max(nv, 1), -1);
@@ -1171,6 +1172,7 @@ int build_device_model(Handle* h) {
   auto addv = [&](const void** slot, const void* p, size_t bytes) { fix.push_back({slot, ar.add(p, bytes)}); };
 #define ADDI(field, vec) addv((const void**)&d.field, vec.data(), vec.size() * sizeof(int))
 #define ADDD(field, vec) addv((const void**)&d.field, vec.data(), vec.size() * sizeof(double))
+#define ADDL(field, vec) addv((const void**)&t.field, vec.data(), vec.size() * sizeof(vec[0]))
   ADDI(body_parent, m.body_parent);
   ADDI(body_jntadr, m.body_jntadr);
   ADDI(body_jntnum, m.body_jntnum);
@@ -1190,24 +1192,12 @@ int build_device_model(Handle* h) {
   ADDI(jnt_limited, m.jnt_limited);
   ADDD(jnt_pos, m.jnt_pos);
   ADDD(jnt_axis, m.jnt_axis);
-  std::vector<double> jnt_unit(m.jnt_axis);
-  for (int j = 0; j < m.njnt; j++) {
-    V3 u = normalized(ld3(&jnt_unit[3 * j]));
-    st3(&jnt_unit[3 * j], u);
-  }
-  ADDD(jnt_unit, jnt_unit);
   ADDD(jnt_range, m.jnt_range);
   ADDD(jnt_stiffness, m.jnt_stiffness);
   ADDD(jnt_springref, m.jnt_springref);
   ADDI(dof_body, m.dof_body);
   ADDI(dof_parent, m.dof_parent);
   ADDD(dof_armature, m.dof_armature);
-  ADDI(dof_limq, dof_limq);
-  ADDD(dof_range, dof_range);
-  ADDI(trunk, trunk);
-  ADDI(limb_adr, limb_adr);
-  ADDI(limb_body, limb_body);
-  ADDI(body_gadr, body_gadr);
   ADDI(dof_block, dof_block);
   ADDI(block_adr, m.dof_blocks);
   ADDI(dofact_adr, dofact_adr);
@@ -1219,12 +1209,6 @@ int build_device_model(Handle* h) {
   ADDD(geom_pos, m.geom_pos);
   ADDD(geom_quat, m.geom_quat);
   ADDI(pair_g, m.pairs);
-  std::vector<int> pair_pack(m.pairs.size() / 2);
-  for (size_t p = 0; p < pair_pack.size(); p++) {
-    int g1 = m.pairs[2 * p], g2 = m.pairs[2 * p + 1];
-    pair_pack[p] = (g1 & 255) | (g2 & 255) << 8 | m.geom_type[g1] << 16 | m.geom_type[g2] << 20;
-  }
-  ADDI(pair_pack, pair_pack);
   ADDI(cam_body, m.cam_body);
   ADDD(cam_pos, m.cam_pos);
   ADDD(cam_quat, m.cam_quat);
@@ -1260,14 +1244,35 @@ int build_device_model(Handle* h) {
   ADDI(hull_nbnum, hull_nbnum);
   ADDI(hull_nb, hull_nb);
   ADDI(hull_seed, hull_seed);
+  ar.host.resize((ar.host.size() + 15) & ~size_t(15));  // staged in 16-byte chunks
+  d.arena_bytes = (int)ar.host.size();
+  // behind the staged part: what only the one- and four-lane substeps read
+  LaneModel& t = h->lm;
+  std::vector<double> jnt_unit(m.jnt_axis);
+  for (int j = 0; j < m.njnt; j++) {
+    V3 u = normalized(ld3(&jnt_unit[3 * j]));
+    st3(&jnt_unit[3 * j], u);
+  }
+  ADDL(jnt_unit, jnt_unit);
+  std::vector<int> pair_pack(m.pairs.size() / 2);
+  for (size_t p = 0; p < pair_pack.size(); p++) {
+    int g1 = m.pairs[2 * p], g2 = m.pairs[2 * p + 1];
+    pair_pack[p] = (g1 & 255) | (g2 & 255) << 8 | m.geom_type[g1] << 16 | m.geom_type[g2] << 20;
+  }
+  ADDL(pair_pack, pair_pack);
+  ADDL(dof_limq, dof_limq);
+  ADDL(dof_range, dof_range);
+  ADDL(trunk, trunk);
+  ADDL(limb_adr, limb_adr);
+  ADDL(limb_body, limb_body);
+  ADDL(body_gadr, body_gadr);
 #undef ADDI
 #undef ADDD
-  ar.host.resize((ar.host.size() + 15) & ~size_t(15));  // staged in 16-byte chunks
+#undef ADDL
   CK(cudaMalloc(&h->d_model, ar.host.size()));
   CK(cudaMemcpy(h->d_model, ar.host.data(), ar.host.size(), cudaMemcpyHostToDevice));
   for (auto& f : fix) *f.slot = (const uint8_t*)h->d_model + f.off;
   d.arena = (const unsigned char*)h->d_model;
-  d.arena_bytes = (int)ar.host.size();
 
   // per-env parameter block
   int off = 0;
@@ -1312,7 +1317,7 @@ int build_device_model(Handle* h) {
     for (int k = 0; k < 3; k++) bp[d.p_bias + 3 * u + k] = m.act_bias[3 * u + k];
   }
   for (int k = 0; k < m.nq; k++) bp[d.p_qpos_reset + k] = m.qpos_reset[k];
-  h->kind = step_kind(m, d);
+  h->kind = step_kind(m, h->lm);
   layouts(m, maxcon, maxrows, h->kind == STEP_QUADS, &h->w, &h->wn, &h->s, &h->k);
   return PG_OK;
 }

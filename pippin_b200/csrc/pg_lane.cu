@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(32) lane_kernel(const __grid_constant__ StepAr
         }
         top++;
         path[top] = b;
-        walk_body(m, b, q, v, cdof, pp, s);
+        walk_body(m, P.t, b, q, v, cdof, pp, s);
       }
     }
     // ------------------------------------------------ passive and actuator forces

@@ -52,7 +52,7 @@ __device__ __forceinline__ void walk_world(const DModel& m, Walk& s) {
 // forward.rs:14-90, 115-164 for body b: on entry s holds its parent's pose,
 // velocity and acceleration, on return its own; its dofs' axes go to cdof.
 // q, v: the env's state; pp: its parameter block.
-__device__ __forceinline__ void walk_body(const DModel& m, int b, const double* q, const double* v, double* cdof,
+__device__ __forceinline__ void walk_body(const DModel& m, const LaneModel& t, int b, const double* q, const double* v, double* cdof,
                                           const double* pp, Walk& s) {
   V3& pos = s.pos;
   Q4& quat = s.quat;
@@ -95,7 +95,7 @@ __device__ __forceinline__ void walk_body(const DModel& m, int b, const double* 
         st6(cdof + 6 * (da + k), Sp{ax, cross(anchor, ax)});
       }
     } else if (type == JNT_HINGE) {
-      V3 jp = ld3(m.jnt_pos + 3 * j), ja = ld3(m.jnt_axis + 3 * j), ju = ld3(m.jnt_unit + 3 * j);
+      V3 jp = ld3(m.jnt_pos + 3 * j), ja = ld3(m.jnt_axis + 3 * j), ju = ld3(t.jnt_unit + 3 * j);
       double sn, cs;
       sincos(0.5 * (q[qa] - m.qpos0[qa]), &sn, &cs);
       M3 rm = turned ? q_mat(quat) : xm;

@@ -21,7 +21,25 @@ constexpr int LANE_DEPTH = 8;   // tree levels below the world
 enum { LC_POS = 0, LC_N = 3, LC_T = 6, LC_MU = 9, LC_D = 10, LC_OFF = 11, LC_MASK = 14, LC_E = 15, LC_P = 18,
        LC_STRIDE = 21 };
 
+// What these kernels read beside DModel: kept out of it, since the phase
+// kernels' blocks each stage DModel and its arrays in shared memory.
+struct LaneModel {
+  // the tree as a trunk (bodies with one child each, from the root down to
+  // the first that branches) and the chains that leave its end (limb_n = -1:
+  // a branch branches again)
+  const int* trunk;     // [trunk_n]
+  const int* limb_adr;  // [limb_n + 1] into limb_body
+  const int* limb_body;
+  const int* body_gadr;  // [nb + 1] first geom of each body (geoms sorted by body)
+  int trunk_n, limb_n, limb_max;  // limb_max: bodies of the longest limb
+  const double* jnt_unit;   // jnt_axis at unit length
+  const int* dof_limq;      // position address of a limited hinge or slide's dof, else -1
+  const double* dof_range;  // [nv][2] its range
+  const int* pair_pack;     // [npair] g1 | g2 << 8 | type1 << 16 | type2 << 20 (models of at most 256 geoms)
+};
+
 struct LaneArgs {
+  LaneModel t;
   // on the device: 0 while the envs' physical parameters are all env 0's,
   // whose block every env then reads (one address for the whole warp); 1 once
   // pg_set_param has written one. Read when the kernel runs, so that a

@@ -78,14 +78,6 @@ struct DModel {
   const int* level_body;
   const int* child_adr;                    // [nb+1] into child_list (children, decreasing id)
   const int* child_list;
-  // the tree as a trunk (bodies with one child each, from the root down to
-  // the first that branches) and the chains that leave its end (limb_n = -1:
-  // a branch branches again)
-  const int* trunk;     // [trunk_n]
-  const int* limb_adr;  // [limb_n + 1] into limb_body
-  const int* limb_body;
-  const int* body_gadr;  // [nb + 1] first geom of each body (geoms sorted by body)
-  int trunk_n, limb_n, limb_max;  // limb_max: bodies of the longest limb
   // ---- joints
   const int* jnt_type;
   const int* jnt_qposadr;
@@ -93,7 +85,6 @@ struct DModel {
   const int* jnt_limited;
   const double* jnt_pos;  // [nj][3]
   const double* jnt_axis;
-  const double* jnt_unit;  // jnt_axis at unit length
   const double* jnt_range;  // [nj][2]
   const double* jnt_stiffness;
   const double* jnt_springref;
@@ -101,8 +92,6 @@ struct DModel {
   const int* dof_body;
   const int* dof_parent;
   const double* dof_armature;
-  const int* dof_limq;      // position address of a limited hinge or slide's dof, else -1
-  const double* dof_range;  // [nv][2] its range
   const int* dof_block;       // block id of each dof
   const int* block_adr;       // [nblock][2] = [start, end)
   const int* dofact_adr;      // [nv+1] actuator contributions per dof, in actuator order
@@ -114,7 +103,6 @@ struct DModel {
   const int* geom_dataid;
   const double* geom_pos;   // [ng][3]
   const double* geom_quat;  // [ng][4]
-  const int* pair_pack;     // [npair] g1 | g2 << 8 | type1 << 16 | type2 << 20 (models of at most 256 geoms)
   const int* pair_g;        // [npair][2] candidate pairs (static filter; masks per env)
   // ---- cameras
   const int* cam_body;

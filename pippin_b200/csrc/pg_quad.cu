@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
       auto geoms = [&](int b, int g0, int step, const Walk& s) {
         if (m.npair > 0)
 #pragma unroll 1
-          for (int g = m.body_gadr[b] + g0; g < m.body_gadr[b + 1]; g += step) {
+          for (int g = P.t.body_gadr[b] + g0; g < P.t.body_gadr[b + 1]; g += step) {
             V3 x, half;
             M3 gm;
             geom_box(m, g, s, pp, &x, &gm, &half);
@@ -301,30 +301,30 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
       Sym I{};
       Sp fr = sp_zero();
 #pragma unroll 1
-      for (int l0 = 0; l0 == 0 || l0 < m.limb_n; l0 += 4) {
+      for (int l0 = 0; l0 == 0 || l0 < P.t.limb_n; l0 += 4) {
         // every lane walks the trunk (the same values), then its limb
         int l = l0 + r;
-        int a0 = l < m.limb_n ? m.limb_adr[l] : 0, a1 = l < m.limb_n ? m.limb_adr[l + 1] : 0;
+        int a0 = l < P.t.limb_n ? P.t.limb_adr[l] : 0, a1 = l < P.t.limb_n ? P.t.limb_adr[l + 1] : 0;
         if (l0 > 0) s = end;
 #pragma unroll 1
-        for (int k = l0 > 0 ? 0 : -m.trunk_n; k < m.limb_max; k++) {
-          if (l0 == 0 && k == 0 && m.limb_n > 4) end = s;
+        for (int k = l0 > 0 ? 0 : -P.t.trunk_n; k < P.t.limb_max; k++) {
+          if (l0 == 0 && k == 0 && P.t.limb_n > 4) end = s;
           if (k < 0 || a0 + k < a1) {
-            int b = k < 0 ? m.trunk[m.trunk_n + k] : m.limb_body[a0 + k];
-            walk_body(m, b, q, v, cdof, pp, s);
+            int b = k < 0 ? P.t.trunk[P.t.trunk_n + k] : P.t.limb_body[a0 + k];
+            walk_body(m, P.t, b, q, v, cdof, pp, s);
             if (k < 0) geoms(b, r, 4, s);
             else geoms(b, 0, 1, s);
-            keep(k < 0 ? tr + 16 * (m.trunk_n + k) : lb + 16 * k, s.I, s.fr);
+            keep(k < 0 ? tr + 16 * (P.t.trunk_n + k) : lb + 16 * k, s.I, s.fr);
           }
           __syncwarp();
         }
         Sym J{};
         Sp jr = sp_zero();
 #pragma unroll 1
-        for (int k = m.limb_max - 1; k >= 0; k--) {
+        for (int k = P.t.limb_max - 1; k >= 0; k--) {
           if (a0 + k < a1) {
             join(lb + 16 * k, J, jr);
-            leave(m.limb_body[a0 + k], J, jr, alive);
+            leave(P.t.limb_body[a0 + k], J, jr, alive);
           }
           __syncwarp();
         }
@@ -343,9 +343,9 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
       fr.ang = V3{quad_sum(fr.ang.x), quad_sum(fr.ang.y), quad_sum(fr.ang.z)};
       fr.lin = V3{quad_sum(fr.lin.x), quad_sum(fr.lin.y), quad_sum(fr.lin.z)};
 #pragma unroll 1
-      for (int k = m.trunk_n - 1; k >= 0; k--) {
+      for (int k = P.t.trunk_n - 1; k >= 0; k--) {
         join(tr + 16 * k, I, fr);
-        leave(m.trunk[k], I, fr, alive && r == 0);
+        leave(P.t.trunk[k], I, fr, alive && r == 0);
       }
       __syncwarp();
     }
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
       for (int k = 0; k < 32 && p0 + 4 * k < m.npair; k++) {
         const int pr = p0 + 4 * k + r;
         bool keep = alive && pr < m.npair;
-        const int pack = m.pair_pack[keep ? pr : 0];
+        const int pack = P.t.pair_pack[keep ? pr : 0];
         const int g1 = pack & 255, g2 = pack >> 8 & 255, ty1 = pack >> 16 & 15, ty2 = pack >> 20;
         if (ty1 != GEOM_PLANE && ty2 != GEOM_PLANE) {
           V3 c1 = ld3(box + 6 * g1), h1 = ld3(box + 6 * g1 + 3), c2 = ld3(box + 6 * g2), h2 = ld3(box + 6 * g2 + 3);
@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
         bool keep = mine != 0;
         const int pr = keep ? p0 + 4 * (__ffs(mine) - 1) + r : 0;
         mine &= mine - 1;
-        const int pack = m.pair_pack[pr];
+        const int pack = P.t.pair_pack[pr];
         const int g1 = pack & 255, g2 = pack >> 8 & 255, ty1 = pack >> 16 & 15, ty2 = pack >> 20;
         const bool flat = (ty1 == GEOM_PLANE) != (ty2 == GEOM_PLANE);
         const int gpl = ty1 == GEOM_PLANE ? g1 : g2, go = ty1 == GEOM_PLANE ? g2 : g1;
@@ -692,11 +692,11 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
           }
 #pragma unroll 1
           for (int k = r; k < nv; k += 4) {
-            int qa = m.dof_limq[k];
+            int qa = P.t.dof_limq[k];
             double lo = 0.0, hi = 0.0;
             if (qa >= 0) {
-              lo = q[qa] - m.dof_range[2 * k];
-              hi = m.dof_range[2 * k + 1] - q[qa];
+              lo = q[qa] - P.t.dof_range[2 * k];
+              hi = P.t.dof_range[2 * k + 1] - q[qa];
             }
             if (lo < 0.0 || hi < 0.0) {
               double sg = lo < 0.0 ? 1.0 : -1.0, sep = lo < 0.0 ? lo : hi;

@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(256, 2) collide_kernel(const __grid_constant__
 // lanes an SM, one wave for 4096 Ant envs. LEARN = false (newton_plain_kernel,
 // launched when the learned start neither predicts nor collects) leaves the
 // learned start's code out of the kernel.
-template <int G, bool LEARN>
+template <int G, bool LEARN, bool PGS>
 __device__ __forceinline__ void newton_phase(const StepArgs& A) {
   extern __shared__ __align__(16) unsigned char smem[];
   const DModel& m = stage_model(A, smem);
@@ -267,7 +267,7 @@ __device__ __forceinline__ void newton_phase(const StepArgs& A) {
       double* v = ws + w.vel;
       double* vpos = v;
       double* qvel = ws + w.qvel;
-      if (m.solver == SOLVER_PGS) {
+      if constexpr (PGS) {
         // forward.rs:366-375: velocities through M + hD, then PGS on them
         // (the factor read in place when it does not live in the workspace)
         const double* lh = w.fac >= 0 ? ws + w.fac : wk + A.k.lh;
@@ -337,11 +337,17 @@ __device__ __forceinline__ void newton_phase(const StepArgs& A) {
 
 template <int G>
 __global__ void __launch_bounds__(256, 2) newton_kernel(const __grid_constant__ StepArgs A) {
-  newton_phase<G, true>(A);
+  newton_phase<G, true, false>(A);
 }
 template <int G>
 __global__ void __launch_bounds__(256, 2) newton_plain_kernel(const __grid_constant__ StepArgs A) {
-  newton_phase<G, false>(A);
+  newton_phase<G, false, false>(A);
+}
+// (in a kernel of its own: with both solvers in one, each solver's loops
+// spilled more)
+template <int G>
+__global__ void __launch_bounds__(256, 2) pgs_kernel(const __grid_constant__ StepArgs A) {
+  newton_phase<G, false, true>(A);
 }
 
 // whether a substep's Newton phase needs the learned start's code
@@ -646,6 +652,7 @@ static const void* kernel_ptr(int which) {
     case K_COLLIDE: return (const void*)collide_kernel<G>;
     case K_NEWTON: return (const void*)newton_kernel<G>;
     case K_NEWTON_PLAIN: return (const void*)newton_plain_kernel<G>;
+    case K_PGS: return (const void*)pgs_kernel<G>;
     case K_SET_CONST: return (const void*)set_const_kernel<G>;
     case K_POSES: return (const void*)poses_kernel<G>;
   }
@@ -668,7 +675,8 @@ size_t kernel_smem(int which, const StepArgs& a, int tiles_per_block) {
       return staged + (size_t)tiles_per_block *
                           (collide_tile_ints(a.m) * sizeof(int) + collide_cache_doubles(a.m) * sizeof(double));
     case K_NEWTON:
-    case K_NEWTON_PLAIN: return staged + (size_t)tiles_per_block * a.wn.stride * sizeof(double);
+    case K_NEWTON_PLAIN:
+    case K_PGS: return staged + (size_t)tiles_per_block * a.wn.stride * sizeof(double);
     default: return staged + (size_t)tiles_per_block * a.w.stride * sizeof(double);
   }
 }
@@ -713,7 +721,8 @@ cudaError_t launch_substep(const StepArgs& a0, const SubstepCfg& c, cudaStream_t
     e = launch_learn(a, a.learn.mode == LEARN_PREDICT, s);
     if (e != cudaSuccess) return e;
   }
-  if (newton_learns(a)) PG_LAUNCH(K_NEWTON, newton_kernel, c.newton, a);
+  if (a.m.solver == SOLVER_PGS) PG_LAUNCH(K_PGS, pgs_kernel, c.newton, a);
+  else if (newton_learns(a)) PG_LAUNCH(K_NEWTON, newton_kernel, c.newton, a);
   else PG_LAUNCH(K_NEWTON_PLAIN, newton_plain_kernel, c.newton, a);
   return cudaSuccess;
 }
@@ -780,7 +789,8 @@ cudaError_t launch_phase(int which, const StepArgs& a0, const LaunchCfg& c, cuda
     case K_SMOOTH: PG_LAUNCH(K_SMOOTH, smooth_kernel, c, a); break;
     case K_COLLIDE: PG_LAUNCH(K_COLLIDE, collide_kernel, c, a); break;
     case K_NEWTON:
-      if (newton_learns(a)) PG_LAUNCH(K_NEWTON, newton_kernel, c, a);
+      if (a.m.solver == SOLVER_PGS) PG_LAUNCH(K_PGS, pgs_kernel, c, a);
+      else if (newton_learns(a)) PG_LAUNCH(K_NEWTON, newton_kernel, c, a);
       else PG_LAUNCH(K_NEWTON_PLAIN, newton_plain_kernel, c, a);
       break;
     default: return cudaErrorInvalidValue;

@@ -801,3 +801,65 @@ def test_full_size_hull_tumble_properties():
     for b in range(m.nq // 7):
         np.testing.assert_allclose(np.linalg.norm(q[:, 7 * b + 3:7 * b + 7], axis=1), 1.0, atol=1e-10)
     _sample_step_parity(g, blob, n, rng.choice(n, 32, replace=False))
+
+
+def _islands_xml(trees):
+    """Free boxes (7-dof trees where "hinged": a second box on a hinge)."""
+    box = '<geom type="box" size=".05 .05 .05" friction="0.7 0.1 0.1"/>'
+    arm = f'<body pos="0.11 0 0"><joint axis="0 0 1" armature="0.01"/>{box}</body>'
+    body = "".join(f'<body pos="{0.4 * k} 0 0.05"><freejoint/>{box}{arm if t == "hinged" else ""}</body>'
+                   for k, t in enumerate(trees))
+    return ('<mujoco><option timestep="0.002" iterations="30"/><worldbody>'
+            f'<geom type="plane" size="5 5 .1" friction="0.7 0.1 0.1"/>{body}</worldbody></mujoco>')
+
+
+@pytest.mark.parametrize("trees,up", [
+    (["box"], [0]),                                     # one tree: the tile
+    (["hinged"], [0]),
+    (["box"] * 2, [0, 1]),                              # joined: the tile, fewer than 16 dofs
+    (["box"] * 3, [0, 1, 2]),                           # joined: the tile
+    (["box"] * 4, [0, 1, 2, None]),                     # all rows in one island: the tile
+    (["box"] * 4, [0, 1, 2, 0]),                        # three quarters of them: the tile
+    (["box"] * 4, [0, 1, 0, 0]),                        # half: a lane each, rows of two trees among them
+    (["box"] * 2, [0, 0]),                              # a lane each, fewer than 16 dofs
+    (["box"] * 6, [0, 1, 2, 0, 0, 0]),
+    (["box"] * 8, [0] * 8),
+    (["hinged", "box", "box"], [0, 0, 0]),              # a tree past six dofs beside two of six
+    (["hinged", "box", "hinged", "box"], [0, 0, 0, 1]),
+])
+def test_pgs_islands(trees, up):
+    """Boxes on the floor (0), on the box before them (1, 2: its height in the
+    stack) or in the air (None): rows of one island, of several, of trees that
+    fit a row's line and of larger ones. A step from states whose depths stay
+    off the slop, where the bias changes branch; PGS stops at the same sweep
+    in both but for rounding (at most one env in twenty)."""
+    n = 24
+    m = mjcf.load_string(_islands_xml(trees))
+    g, o = CudaPhysics(mjcf.to_blob(m), n), Oracle(mjcf.to_blob(m), n, threads=4)
+    for sim in (g, o):
+        sim.set_solver(kind=1)
+    rng = np.random.default_rng(len(trees) + 10 * sum(u or 0 for u in up))
+    q = np.tile(np.array(m.qpos0), (n, 1))
+    free = [m.jnt_qposadr[j] for j in range(m.njnt) if m.jnt_type[j] == mjcf.JNT_FREE]
+    for k, (a, u) in enumerate(zip(free, up)):
+        q[:, a] = 0.4 * k + rng.uniform(-0.01, 0.01, n) if not u else q[:, free[k - 1]] + rng.uniform(-0.01, 0.01, n)
+        q[:, a + 2] = (5.0 if u is None else 0.05 + 0.1 * u - 0.0015 * (u + 1)) + rng.uniform(-2e-4, 2e-4, n)
+        w = np.array([1.0, 0, 0, 0]) + rng.uniform(-0.002, 0.002, (n, 4))  # (off the ties of aligned faces)
+        q[:, a + 3:a + 7] = w / np.linalg.norm(w, axis=1, keepdims=True)
+    v = rng.normal(0, 0.2, (n, m.nv))
+    g.set(Field.QPOS, range(n), q)
+    g.set(Field.QVEL, range(n), v)
+    o.set(QPOS, q)
+    o.set(QVEL, v)
+    g.step(range(n), 1)
+    o.step(0, n, 1)
+    sg, so = g.stats(), o.stats()
+    np.testing.assert_array_equal(sg["nrows"], so["nrows"])
+    assert (sg["nrows"] > 0).all() and not sg["status"].any()
+    same = sg["iters"] == so["iters"]
+    assert same.sum() >= 0.95 * n
+    for fg, fo in ((Field.QACC, QACC), (Field.QVEL, QVEL), (Field.QPOS, QPOS)):
+        a, b = g.get(fg, range(n)), o.get(fo)
+        for e in range(n):
+            if same[e]:
+                assert rel(a[e], b[e]) < TOL_STEP, (e, fg, rel(a[e], b[e]))

@@ -90,14 +90,15 @@ extern "C" int pg_step_static(pg_handle* h, int64_t start, int64_t end, int64_t 
   int rc = pg::internal_step_args(h, start, end, nstep, &a, &cfg, &stream, &device);
   if (rc != PG_OK) return rc;
   if (end == start || nstep == 0) return PG_OK;
-  // one or four lanes an env need no tile scratch at all
-  if (pg::internal_step_lanes(h, a, start, end, nstep, &rc)) return rc;
   unsigned char* base = nullptr;  // internal_step_args made the handle's device current
   if ((rc = scratch_address(&base)) != PG_OK) return rc;
   // only the Newton phase uses tile scratch: its grid is capped by the array
   pg::LaunchCfg& nc = cfg.newton;
   int64_t tiles = 0;
   if ((rc = pg_static_tiles((size_t)a.s.stride * sizeof(double), nc.tiles_per_block, &tiles)) != PG_OK) return rc;
+  // one or four lanes an env need no tile scratch at all (a model whose tiles
+  // do not fit it is rejected all the same: whether they run it may change)
+  if (pg::internal_step_lanes(h, a, start, end, nstep, &rc)) return rc;
   nc.blocks = (int)std::min<int64_t>((int64_t)nc.blocks, tiles / nc.tiles_per_block);
   a.queue = reinterpret_cast<int*>(base);
   a.order = nullptr;  // envs in index order: an order array would need memory per env

@@ -144,3 +144,18 @@ def test_steps_that_cannot_be_captured_are_refused(name):
         p.step(range(n), 1)
         p.synchronize()
     np.testing.assert_array_equal(a.get(Field.QACC, range(n)), b.get(Field.QACC, range(n)))
+
+
+def test_static_steps_refuse_models_past_their_scratch():
+    """Four links of 28 masked-out boxes each: 2352 candidate pairs, whose rows
+    take 4 MB a tile, 17 a block. The step needs no tile while nothing can
+    touch, but may need one for the next call; pg_step takes the model."""
+    box = "".join(f'<geom type="box" size="0.01 0.01 0.01" pos="0 0 {0.03 * i:.2f}" contype="0" conaffinity="0"/>'
+                  for i in range(28))
+    link = f'<body pos="0.1 0 0"><joint axis="0 1 0"/>{box}'
+    p = CudaPhysics(f'<mujoco><worldbody>{4 * link}{4 * "</body>"}</worldbody></mujoco>', 2)
+    assert p.step_lanes() == 1
+    assert _native.load().pg_step_static(p._h, 0, 2, 1) == 4  # PG_ERR_UNSUPPORTED
+    assert "scratch" in _native.last_error()
+    p.step(range(2), 1)
+    p.synchronize()

@@ -146,8 +146,8 @@ int pg_step_device(pg_handle* h, int64_t start, int64_t end, int64_t nstep, cons
  * first call on a device also loads the library's device image there, so make
  * it before any stream capture (pg_step and pg_step_device refuse to be
  * captured: they replay graphs of their own). A captured call keeps the solver
- * settings of its capture and reads the parameters of its replay. All calls share the array and keep its last
- * contents: calls that overlap on the GPU race. Stream-ordered like pg_step. */
+ * settings of its capture and reads the parameters of its replay. All calls
+ * share the array and keep its last contents: calls that overlap on the GPU race. Stream-ordered like pg_step. */
 int pg_step_static(pg_handle* h, int64_t start, int64_t end, int64_t nstep);
 
 /* Batch::rollout (crates/pippin/src/batch.rs:46-59): ctrl is
@@ -236,9 +236,10 @@ int pg_invweight(pg_handle* h, int64_t env, double* body, double* dof);
 
 /* Launch shape: lanes per env (8, 16, 32) and envs per block; 0 = keep.
  * Naming a shape makes pg_step run the phase kernels in it where it would run
- * the substep in one kernel. pg_autotune times the candidate shapes on the
- * current state (which it saves and restores) and keeps the fastest; it has
- * nothing to do for a handle whose substep is one kernel. */
+ * the substep in one kernel, until a call that names none (0, 0). pg_autotune
+ * times the candidate shapes of the phase kernels on the current state (which
+ * it saves and restores) and keeps the fastest; which kernel pg_step runs stays
+ * as it is. */
 int pg_set_launch(pg_handle* h, int lanes_per_env, int envs_per_block);
 int pg_get_launch(const pg_handle* h, int* lanes_per_env, int* envs_per_block, int* blocks);
 int pg_autotune(pg_handle* h, int64_t nstep);

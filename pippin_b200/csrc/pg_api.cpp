@@ -1939,9 +1939,11 @@ int pg_set_launch(pg_handle* h, int lanes_per_env, int envs_per_block) {
     if (envs_per_block > 0) p->tiles_per_block = envs_per_block;
   }
   CK(cudaSetDevice(h->device));
-  // a caller that names a shape gets the phase kernels in it
-  if (lanes_per_env > 0 || envs_per_block > 0) h->forced_shape = true;
-  return apply_cfg(h, c);
+  if (int rc = apply_cfg(h, c)) return rc;
+  // a caller that names a shape gets the phase kernels in it, until one that
+  // names none
+  h->forced_shape = lanes_per_env > 0 || envs_per_block > 0;
+  return PG_OK;
 }
 
 int pg_get_launch(const pg_handle* h, int* lanes_per_env, int* envs_per_block, int* blocks) {
@@ -1973,7 +1975,6 @@ int pg_autotune(pg_handle* h, int64_t nstep) {
   if (h->n == 0) return PG_OK;
   if (nstep < 1) nstep = 1;
   CK(cudaSetDevice(h->device));
-  if (use_lanes(h)) return PG_OK;  // the one-lane-per-env substep has no shape to search
   const HostModel& m = h->hm;
   size_t n = h->n;
   // save the state the trial steps will overwrite

@@ -159,3 +159,29 @@ def test_static_steps_refuse_models_past_their_scratch():
     assert "scratch" in _native.last_error()
     p.step(range(2), 1)
     p.synchronize()
+
+
+def test_set_launch_and_autotune_leave_the_kernel_to_the_caller():
+    n = 2048
+    p = CudaPhysics(scenes.ant_xml(), n)
+    assert p.step_lanes() == 4
+    with pytest.raises(PhysicsError):
+        p.set_launch(64, 4)  # refused: nothing changes
+    assert p.step_lanes() == 4
+    p.set_launch(32, 1)
+    assert p.step_lanes() == 0
+    p.set_launch()  # names no shape any more
+    assert p.step_lanes() == 4
+    shapes = p.phase_launch()
+    assert all(s[:2] == (32, 1) for s in shapes.values())
+    # the phase kernels' shapes are searched all the same: PGS, the learned
+    # start and time_phases run in them
+    rng = np.random.default_rng(0)
+    p.set(Field.QVEL, range(n), rng.normal(0, 1, (n, 14)))
+    p.step(range(n), 20)
+    state = {f: p.get(f, range(n)) for f in Field}
+    p.autotune()
+    assert p.step_lanes() == 4
+    assert any(s[:2] != (32, 1) for s in p.phase_launch().values())
+    for f in Field:
+        np.testing.assert_array_equal(p.get(f, range(n)), state[f])

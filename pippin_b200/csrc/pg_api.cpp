@@ -1754,10 +1754,18 @@ int pg_get_param(pg_handle* h, int param, int64_t id, int64_t start, int64_t end
     return fail(PG_ERR_INVALID, std::string(param_name(param)) + ": id " + std::to_string(id) + " out of range");
   if (end == start) return PG_OK;
   CK(cudaSetDevice(h->device));
-  // gathered on the device: the whole blocks (3.4 KB an Ant env) took 3.5 ms
-  // to bring back for 8192 envs, one parameter's values a few microseconds
-  if ((rc = grow(h, h->b_vals, sizeof(double) * len))) return rc;
   int step = 1, off = param_offset(h->dm, param, id, &step);
+  // a few envs' blocks (3.4 KB an Ant env) come back whole, without a launch
+  // (1 env 18.7 us, gathered 22.7; 0.6 us more each further env)
+  if (end - start <= 4) {
+    std::vector<double> blk;
+    if ((rc = read_params(h, start, end, blk))) return rc;
+    for (int64_t k = 0; k < (end - start) * w; k++) out[k] = blk[k / w * h->dm.pstride + off + k % w * step];
+    return PG_OK;
+  }
+  // gathered on the device: the whole blocks took 3.5 ms to bring back for
+  // 8192 envs, one parameter's values a few microseconds
+  if ((rc = grow(h, h->b_vals, sizeof(double) * len))) return rc;
   CK(launch_read_param(h->params + start * h->dm.pstride, h->dm.pstride, end - start, off, w, step, (double*)h->b_vals.p,
                        h->stream));
   return copy_rows_d2h(h, out, (const double*)h->b_vals.p, 0, end - start, w);

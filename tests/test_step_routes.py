@@ -185,3 +185,27 @@ def test_set_launch_and_autotune_leave_the_kernel_to_the_caller():
     assert any(s[:2] != (32, 1) for s in p.phase_launch().values())
     for f in Field:
         np.testing.assert_array_equal(p.get(f, range(n)), state[f])
+
+
+@pytest.mark.parametrize("count", [1, 2, 3, 4, 5, 33])
+def test_get_param_returns_what_set_param_wrote(count):
+    n, s0 = 70, 30
+    p = CudaPhysics(scenes.ant_xml(), n)
+    rng = np.random.default_rng(count)
+    for pid in Param:
+        w = p.param_width(pid)
+        if pid == Param.QPOS0:
+            val = np.tile(p.get_param(pid, 0, range(1)), (count, 1)) + 0.01 * rng.random((count, 1))
+            val[:, 3:7] = [1.0, 0.0, 0.0, 0.0]
+        elif pid in (Param.GEOM_CONTYPE, Param.GEOM_CONAFFINITY):
+            val = rng.integers(0, 8, (count, w)).astype(float)
+        elif pid == Param.BODY_INERTIA:
+            val = 1.0 + 0.1 * rng.random((count, w))
+        else:  # (colours are kept in 32 bits)
+            val = (0.5 + rng.random((count, w))).astype(np.float32).astype(float)
+        before = p.get_param(pid, 0 if pid == Param.QPOS0 else 1, range(n))
+        elem = 0 if pid == Param.QPOS0 else 1
+        p.set_param(pid, elem, range(s0, s0 + count), val)
+        np.testing.assert_array_equal(p.get_param(pid, elem, range(s0, s0 + count)), val)
+        for e in (s0 - 1, s0 + count):  # the neighbours keep theirs
+            np.testing.assert_array_equal(p.get_param(pid, elem, range(e, e + 1))[0], before[e])

@@ -727,9 +727,11 @@ int set_const_range(Handle* h, int64_t start, int64_t end) {
 // Whether the handle's substeps run on one or four lanes an env. Measured
 // against the three phase kernels (us a substep, single-substep calls, 4 / 512
 // / 4096 / 16384 envs):
-//   one lane, models without constraint rows: pendulum 11 / 13 / 13 / 13
-//   against 45 / 45 / 52 / 118, cartpole 17 / 20 / 21 / 21 against 56 / 54 /
-//   63 / 163. With rows a lane's Newton loses to the phase kernels in the
+//   one lane, models without constraint rows, of at most 8 dofs: pendulum 11 /
+//   13 / 13 / 13 against 45 / 45 / 52 / 118, cartpole 17 / 20 / 21 / 21 against
+//   56 / 54 / 63 / 163. Past 8 dofs a lane's matrix spills: two arms of 15
+//   dofs 86 / 141 / 140 / 143 (1 / 512 / 4096 / 16384 envs, with the wait)
+//   against 83 / 83 / 160 / 402; four lanes 74 / 76 / 77 / 158. With rows a lane's Newton loses to the phase kernels in the
 //   middle of the range (a 6-hinge chain: 62 / 145 / 200 / 259 against 94 /
 //   130 / 167 / 446), so such models go elsewhere;
 //   four lanes, one tree with rows possible: Ant 65 / 95 / 113 / 217 against
@@ -922,10 +924,10 @@ bool pair_masked(const HostModel& m, size_t p) {
   return !(m.geom_contype[a] & m.geom_conaffinity[b]) && !(m.geom_contype[b] & m.geom_conaffinity[a]);
 }
 // The substep a model's Newton steps take (STEP_*): see the rule's figures at
-// the definition of use_lanes. Both kernels hold one tree of at most 16 dofs
-// and need the bodies depth first and explicit damping.
+// the definition of use_lanes. Both kernels hold one tree (of at most 16 dofs,
+// 8 on one lane) and need the bodies depth first and explicit damping.
 int step_kind(const HostModel& m, const LaneModel& t) {
-  if (m.nv < 1 || m.nv > LANE_NV || m.nq > LANE_NQ || m.dof_blocks.size() != 2 || m.neq > 0 || m.integrator != 0)
+  if (m.nv < 1 || m.nv > QUAD_NV || m.nq > LANE_NQ || m.dof_blocks.size() != 2 || m.neq > 0 || m.integrator != 0)
     return STEP_PHASES;
   std::vector<int> path = {0};
   for (int b = 1; b < m.nbody; b++) {
@@ -936,7 +938,7 @@ int step_kind(const HostModel& m, const LaneModel& t) {
   bool rows = false;
   for (int j = 0; j < m.njnt; j++) rows |= m.jnt_limited[j] && (m.jnt_type[j] == JNT_HINGE || m.jnt_type[j] == JNT_SLIDE);
   for (size_t p = 0; 2 * p + 1 < m.pairs.size(); p++) rows |= !pair_masked(m, p);
-  if (!rows && t.limb_n < 3) return STEP_LANES;
+  if (!rows && t.limb_n < 3 && m.nv <= LANE_NV) return STEP_LANES;
   // four lanes: limbs that are chains, primitive pairs, at most one violated
   // side a limit, geoms in body order
   if (t.limb_n < 0 || t.trunk_n > LANE_DEPTH || t.limb_max > LANE_DEPTH || m.nu > QUAD_NU || m.ngeom > LANE_GEOM)

@@ -1,4 +1,4 @@
-// The whole substep with one lane per environment, for models of at most 16
+// The whole substep with one lane per environment, for models of at most 8
 // dofs in one tree that can have no constraint rows (no limits, every pair
 // masked out): control tasks and arms.
 //
@@ -295,8 +295,7 @@ cudaError_t launch_lane(const StepArgs& a, const LaneArgs& p, cudaStream_t s) {
   int64_t warps = ((int64_t)a.count + p.lanes - 1) / p.lanes;
   if (warps <= 0) return cudaSuccess;
   if (a.m.nv <= 4) lane_kernel<4><<<(unsigned)warps, 32, 0, s>>>(a, p);
-  else if (a.m.nv <= 8) lane_kernel<8><<<(unsigned)warps, 32, 0, s>>>(a, p);
-  else lane_kernel<16><<<(unsigned)warps, 32, 0, s>>>(a, p);
+  else lane_kernel<8><<<(unsigned)warps, 32, 0, s>>>(a, p);
   return cudaGetLastError();
 }
 

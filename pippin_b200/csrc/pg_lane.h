@@ -10,7 +10,8 @@ namespace pg {
 // lane an env (no constraint rows possible), or four
 enum { STEP_PHASES = 0, STEP_LANES = 1, STEP_QUADS = 2 };
 // limits of the models the lane and quad kernels take (sizes of its per-lane arrays)
-constexpr int LANE_NV = 16;     // dofs
+constexpr int LANE_NV = 8;      // dofs (lane)
+constexpr int QUAD_NV = 16;     // dofs (quad)
 constexpr int LANE_NQ = 24;     // positions
 constexpr int LANE_GEOM = 32;   // geoms
 constexpr int QUAD_NU = 32;     // actuators (quad)

@@ -11,7 +11,7 @@ Newton exit leave four digits more).
 import numpy as np
 import pytest
 
-from oracle.oracle import CTRL, QACC, QPOS, QVEL, Oracle
+from oracle.oracle import CTRL, QACC, QFRC_APPLIED, QPOS, QVEL, Oracle
 from pippin_b200 import CudaPhysics, Field, Param, WarmStart, mjcf, scenes
 
 pytestmark = pytest.mark.gpu
@@ -296,3 +296,52 @@ def test_body_frames_turned_by_less_than_the_real_part_shows(name):
     g.set(Field.QPOS, range(n), q)
     g.set(Field.QVEL, range(n), v)
     _oracle_step(g, o, n, TOL)
+
+
+def _arms(arms, depth, fork=0, root=True):
+    """Contact-free arms of `depth` hinges off one body, `fork` more bodies at
+    the end of each."""
+    g = '<geom type="capsule" fromto="0 0 0 0.12 0 0" size="0.035" contype="0" conaffinity="0"/>'
+
+    def link(k, inner):
+        axis = ["0 0 1", "0 1 0", "1 0 0"][k % 3]
+        return (f'<body pos="0.12 0.02 0" euler="0 {5 * (k % 3)} {4 * k}"><joint axis="{axis}" armature="0.02" '
+                f'damping="{0.1 * (k % 2)}"/>{g}{inner}</body>')
+
+    def arm(a, k):
+        return "".join(link(a + k + f, "") for f in range(fork)) if k == depth else link(a + k, arm(a, k + 1))
+
+    body = "".join(arm(a, 0) for a in range(arms))
+    joint = '<joint axis="0 0 1" armature="0.1"/>' if root else ""
+    return f'<mujoco>{OPT}<worldbody><body pos="0 0 1">{joint}{g}{body}</body></worldbody></mujoco>'
+
+
+FREE = {  # dofs, lanes
+    "arm_of_7": (_arms(1, 7, root=False), 7, 1),
+    "two_arms_and_root_9": (_arms(2, 4), 9, 4),
+    "two_arms_15": (_arms(2, 7), 15, 4),
+    "three_arms_16": (_arms(3, 5), 16, 4),
+    "forks_7": (_arms(2, 1, fork=2), 7, 1),
+    "forks_13": (_arms(4, 1, fork=2), 13, 0),
+}
+
+
+@pytest.mark.parametrize("name", list(FREE))
+@pytest.mark.parametrize("n", [1, 33, 700, 5001])
+def test_models_without_rows(name, n):
+    """One lane up to 8 dofs, four lanes up to 16 where the branches are
+    chains, the phase kernels beyond."""
+    xml, dofs, lanes = FREE[name]
+    m = mjcf.load_string(xml)
+    assert m.nv == dofs
+    blob = mjcf.to_blob(m)
+    g, o = CudaPhysics(blob, n), Oracle(blob, n, threads=8)
+    assert g.step_lanes() == lanes
+    rng = np.random.default_rng(n)
+    q, v = _states(m, n, rng)
+    g.set(Field.QPOS, range(n), q)
+    g.set(Field.QVEL, range(n), v)
+    g.set(Field.QFRC_APPLIED, range(n), rng.normal(0, 1, (n, m.nv)))
+    o.set(QFRC_APPLIED, g.get(Field.QFRC_APPLIED, range(n)))
+    for _ in range(3):
+        assert not _oracle_step(g, o, n, TOL)["nrows"].any()

@@ -345,3 +345,49 @@ def test_models_without_rows(name, n):
     o.set(QFRC_APPLIED, g.get(Field.QFRC_APPLIED, range(n)))
     for _ in range(3):
         assert not _oracle_step(g, o, n, TOL)["nrows"].any()
+
+
+@pytest.mark.parametrize("name", ["hinge_3_limbs", "free_3_limbs", "free_5_limbs"])
+@pytest.mark.parametrize("n", [2501, 9001])
+def test_full_warps_and_blocks(name, n):
+    """Batches of four and eight envs a warp, the last warp ragged, up to
+    eight warps a block, for each size of the matrix but Ant's."""
+    m = mjcf.load_string(MODELS[name])
+    blob = mjcf.to_blob(m)
+    g, o = CudaPhysics(blob, n), Oracle(blob, n, threads=8)
+    assert g.step_lanes() == 4
+    for sim in (g, o):
+        sim.set_solver(tolerance=1e-10, iterations=30)
+    q, v = _states(m, n, np.random.default_rng(n))
+    g.set(Field.QPOS, range(n), q)
+    g.set(Field.QVEL, range(n), v)
+    for _ in range(2):
+        rows = _oracle_step(g, o, n, TOL)["nrows"]
+    assert rows.any()
+
+
+def test_more_than_128_candidate_pairs():
+    """A second pass of the pair loop, whose pairs (limb against limb, after
+    those of the floor and the trunk) touch while earlier ones do as well."""
+    n = 60
+    extra = "".join(f'<geom type="sphere" size="0.03" pos="{0.02 * k - 0.13:.2f} 0 0.08"/>' for k in range(14))
+    xml = _star(5, geoms=("sphere",)).replace('density="400"/>', f'density="400"/>{extra}').replace('size="0.07"/>', 'size="0.22"/>')
+    m = mjcf.load_string(xml)
+    blob = mjcf.to_blob(m)
+    ng = len(m.geom_type)
+    assert ng <= 32
+    g, o = CudaPhysics(blob, n), Oracle(blob, n, threads=8)
+    assert g.step_lanes() == 4
+    for sim in (g, o):
+        sim.set_solver(tolerance=1e-10, iterations=30)
+    q, v = _states(m, n, np.random.default_rng(6))
+    g.set(Field.QPOS, range(n), q)
+    g.set(Field.QVEL, range(n), v)
+    early = late = 0
+    for _ in range(3):
+        for e in range(n):
+            pairs = [(int(c[10]), int(c[11])) for c in g.debug_forward(e)["contacts"]]
+            late += any(min(p) >= ng - 4 for p in pairs)  # between the last two limbs
+            early += any(min(p) == 0 for p in pairs)      # with the floor
+        _oracle_step(g, o, n, TOL)
+    assert early and late

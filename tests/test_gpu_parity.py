@@ -92,16 +92,30 @@ def test_forward_parity(name):
             assert rel(cg[:, :10], co[:, :10]) < TOL_MC, e
 
 
+# Ant steps in one kernel, four lanes an env, unless a shape of the phase
+# kernels is named: both routes hold the same contracts
+both_routes = pytest.mark.parametrize("lanes", [4, 0], ids=["one_kernel", "phase_kernels"])
+
+
+def take_route(lanes, *handles):
+    for p in handles:
+        if lanes == 0:
+            p.set_launch(*p.launch()[:2])
+        assert p.step_lanes() == lanes
+
+
 def _copy_state(src_g, dst_o, n):
     for fg, fo in ((Field.QPOS, QPOS), (Field.QVEL, QVEL), (Field.QACC, QACC), (Field.CTRL, CTRL)):
         dst_o.set(fo, src_g.get(fg, range(n)))
 
 
-def test_ant_step_parity_on_identical_states():
+@both_routes
+def test_ant_step_parity_on_identical_states(lanes):
     """Per-step Newton output on identical input states (config 1 setup,
     tolerance 1e-10), through falls, ground contact and joint limits."""
     n, T = 64, 120
     m, g, o = pair(scenes.ant_xml(), n, tolerance=1e-10)
+    take_route(lanes, g)
     rng = np.random.default_rng(0)
     q, v = random_state(m, n, rng)
     g.set(Field.QPOS, range(n), q)
@@ -502,13 +516,15 @@ def test_reset_keeps_qacc_and_restores_state():
     np.testing.assert_array_equal(g.get(Field.QACC, range(n)), qacc)
 
 
-def test_subranges_step_like_the_whole():
+@both_routes
+def test_subranges_step_like_the_whole(lanes):
     """Stepping halves separately equals stepping all envs (the async
     pipeline steps groups, backends_agree.rs:12-14)."""
     n = 32
     m = mjcf.load_string(scenes.ant_xml())
     blob = mjcf.to_blob(m)
     a, b = CudaPhysics(blob, n), CudaPhysics(blob, n)
+    take_route(lanes, a, b)
     rng = np.random.default_rng(4)
     q, v = random_state(m, n, rng)
     for p in (a, b):
@@ -520,19 +536,22 @@ def test_subranges_step_like_the_whole():
     np.testing.assert_array_equal(a.get(Field.QPOS, range(n)), b.get(Field.QPOS, range(n)))
 
 
-def test_queued_newton_order_steps_like_one_wave():
-    """With more envs than the Newton grid has tiles, the Newton phase takes
-    envs in the order the collision phase wrote (envs with contacts first);
-    with a tile per env it takes them in index order. Both must give every
-    env the same bits: all 12000 envs at once against ranges of 2000 (one
+@both_routes
+def test_queued_newton_order_steps_like_one_wave(lanes):
+    """In the phase kernels, with more envs than the Newton grid has tiles, the
+    Newton phase takes envs in the order the collision phase wrote (envs with
+    contacts first); with a tile per env it takes them in index order. In one
+    kernel the two take other envs a warp and warps a block. Both must give
+    every env the same bits: all 12000 envs at once against ranges of 2000 (one
     wave each), for pg_step and for pg_rollout (whose per-substep qpos goes
     to the env's own row of the output)."""
     n, t = 12000, 6
     m = mjcf.load_string(scenes.ant_xml(tolerance=1e-10))
     blob = mjcf.to_blob(m)
     a, b = CudaPhysics(blob, n), CudaPhysics(blob, n)
-    lanes, per_block, blocks = a.phase_launch()["newton"]
-    assert per_block * blocks < n  # the queued, ordered path
+    take_route(lanes, a, b)
+    _, per_block, blocks = a.phase_launch()["newton"]
+    assert lanes or per_block * blocks < n  # the queued, ordered path
     rng = np.random.default_rng(12)
     q, v = random_state(m, n, rng, qnoise=0.3, vscale=0.5)
     q[:, 2] = rng.uniform(0.2, 0.9, n)  # torso heights: some envs touch the floor, others fly
@@ -553,11 +572,13 @@ def test_queued_newton_order_steps_like_one_wave():
     np.testing.assert_array_equal(out_a, out_b)
 
 
-def test_rollout_matches_step_loop():
+@both_routes
+def test_rollout_matches_step_loop(lanes):
     n, t = 8, 30
     m = mjcf.load_string(scenes.ant_xml())
     blob = mjcf.to_blob(m)
     a, b = CudaPhysics(blob, n), CudaPhysics(blob, n)
+    take_route(lanes, a, b)
     ctrl = np.sin(np.arange(n * t * m.nu) * 0.37).reshape(n, t, m.nu)
     out = a.rollout(ctrl)
     for k in range(t):

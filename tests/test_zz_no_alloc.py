@@ -8,7 +8,9 @@ from the same state; one steps with pg_step, the other with pg_step_static
 through the C-ABI, twice in a row (the second call finds the array holding the
 first call's contents), and the states must agree within the parity
 tolerance of the other GPU tests. The batch is larger than the number of envs
-the static scratch steps at once, so the work loop runs several rounds.
+the static scratch steps at once, so the work loop runs several rounds. (Ant
+takes the scratch with a launch shape of the phase kernels named, their
+register Newton; its one-kernel step needs none.)
 """
 import ctypes as C
 
@@ -26,12 +28,17 @@ def rel(a, b):
     return float(np.max(np.abs(a - b)) / max(float(np.max(np.abs(b))), 1.0))
 
 
-def test_static_scratch_step_matches_pg_step():
+@pytest.mark.parametrize("lanes", [4, 0], ids=["one_kernel", "phase_kernels"])
+def test_static_scratch_step_matches_pg_step(lanes):
     L = _native.load()
     n = 1024
     m = mjcf.load_string(scenes.ant_xml(tolerance=1e-10))
     blob = mjcf.to_blob(m)
     ref, stat = CudaPhysics(blob, n), CudaPhysics(blob, n)
+    for p in (ref, stat):
+        if lanes == 0:
+            p.set_launch(*p.launch()[:2])
+        assert p.step_lanes() == lanes
     rng = np.random.default_rng(11)
     q = np.tile(np.array(m.qpos0), (n, 1)) + rng.uniform(-0.1, 0.1, (n, m.nq))
     v = rng.normal(0, 0.1, (n, m.nv))

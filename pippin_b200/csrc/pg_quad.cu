@@ -77,7 +77,8 @@ struct QuadLayout {
 // earlier one, so the pivots are scalar ones (one division for both). A 2 x 2 inverse in their place is not backward stable, and H's rows
 // are nearly dependent wherever contacts are much stiffer than M: with
 // impratio 100, or solimp up to 0.9999, it cost two digits of qacc. False if a
-// pivot is not positive (the same on the env's four lanes).
+// pivot is not positive (the same on the env's four lanes). (Sums of products
+// are written so that each product is one FMA.)
 template <int N>
 __device__ __forceinline__ bool quad_factor_solve(double (&h)[(N + 3) / 4][N], double (&x)[(N + 3) / 4], double* buf, int r) {
   static_assert(N % 2 == 0, "two rows a step");
@@ -121,7 +122,7 @@ __device__ __forceinline__ bool quad_factor_solve(double (&h)[(N + 3) / 4][N], d
           l0[t] = a0 * i0;
           l1[t] = a1 * i1;
         }
-        x[t] -= l0[t] * x0 + l1[t] * x1;
+        x[t] = (x[t] - l1[t] * x1) - l0[t] * x0;
       }
     }
     __syncwarp();
@@ -130,7 +131,7 @@ __device__ __forceinline__ bool quad_factor_solve(double (&h)[(N + 3) / 4][N], d
       const double e0 = r0[j], e1 = r1[j];
 #pragma unroll
       for (int t = 0; t < T; t++)
-        if (4 * t < k0 && j <= 4 * t + 3) h[t][j] -= l0[t] * e0 + l1[t] * e1;
+        if (4 * t < k0 && j <= 4 * t + 3) h[t][j] = (h[t][j] - l1[t] * e1) - l0[t] * e0;
     }
   }
   // each pair of unknowns in turn, its products with the later rows summed in s
@@ -148,7 +149,7 @@ __device__ __forceinline__ bool quad_factor_solve(double (&h)[(N + 3) / 4][N], d
     const double y1 = __shfl_sync(FULL, y, k0 % 4 + 1, 4);
 #pragma unroll
     for (int t = tk; t < T; t++)
-      if (4 * t + r > k0 + 1) s[t] += h[t][k0] * y0 + h[t][k0 + 1] * y1;
+      if (4 * t + r > k0 + 1) s[t] = (s[t] + h[t][k0] * y0) + h[t][k0 + 1] * y1;
   }
   __syncwarp();
   return ok;

@@ -1453,9 +1453,14 @@ int pg_create(const void* blob, size_t bytes, int64_t n_envs, int device, pg_han
   int gc = npair > 16 ? 32 : (npair > 8 ? 16 : 8);
   // general convex pairs share their faces and edges out over the lanes: for
   // polytopes of up to 64 vertices 16 lanes are enough, and twice the envs
-  // fit (4096 tabletop envs 857 -> 575 us, hulls of up to 32 vertices 328 ->
-  // 334); larger hulls keep 32
-  if (h->dm.gen_vmax > 0 && h->dm.gen_vmax <= HULL_SCAN_BELOW) gc = std::min(gc, 16);
+  // fit (collision phase, 4096 tabletop envs 696 -> 514 us, hulls of up to 32
+  // vertices 275 -> 258); larger hulls keep 32. So do models of many pairs,
+  // whose broad phase takes a lane a pair, while all envs fit in one wave of
+  // 32-lane tiles (16 an SM): 60 / 512 / 1024 tabletop envs (243 pairs) 185 /
+  // 215 / 285 us on 32 lanes, 230 / 262 / 335 on 16; the hulls (36 pairs) 78 /
+  // 82 / 102 and 73 / 76 / 97
+  const bool one_wave = n_envs <= 16ll * h->sm_count;
+  if (h->dm.gen_vmax > 0 && h->dm.gen_vmax <= HULL_SCAN_BELOW && (npair <= 64 || !one_wave)) gc = std::min(gc, 16);
   SubstepCfg want{{g, 4, 0}, {gc, 4, 0}, {g, 4, 0}};
   {
     StepArgs a = make_args(h.get());

@@ -209,3 +209,14 @@ def test_get_param_returns_what_set_param_wrote(count):
         np.testing.assert_array_equal(p.get_param(pid, elem, range(s0, s0 + count)), val)
         for e in (s0 - 1, s0 + count):  # the neighbours keep theirs
             np.testing.assert_array_equal(p.get_param(pid, elem, range(e, e + 1))[0], before[e])
+
+
+def test_collision_lanes_by_pairs_and_batch():
+    """Models of many pairs take 32 lanes an env in the collision phase while
+    one wave holds the batch, 16 beyond; models of few pairs 16."""
+    tabletop = scenes.tabletop(2).xml
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for xml, n, lanes in ((tabletop, 60, 32), (tabletop, 16 * sms, 32), (tabletop, 16 * sms + 1, 16),
+                          (scenes.hull_tumble_xml(), 60, 16), (scenes.hull_tumble_xml(), 16 * sms + 1, 16)):
+        with CudaPhysics(xml, n) as p:
+            assert p.phase_launch()["collide"][0] == lanes, n

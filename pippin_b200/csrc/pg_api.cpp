@@ -661,7 +661,10 @@ int choose_grid(Handle* h, int phase, const LaunchCfg& want, LaunchCfg* out) {
   StepArgs a = make_args(h);
   std::vector<int> kinds = {phase};
   if (phase == K_SMOOTH) kinds = {K_SMOOTH, K_SET_CONST, K_POSES};
-  if (phase == K_NEWTON) kinds = {K_NEWTON, K_NEWTON_PLAIN, K_PGS};  // with and without the learned start's code
+  if (phase == K_NEWTON) {
+    kinds = {K_NEWTON, K_NEWTON_PLAIN};  // with and without the learned start's code
+    if (h->dm.solver == SOLVER_PGS) kinds.push_back(K_PGS);  // (its code loads with the first handle that steps PGS)
+  }
   int per_sm = 0;
   for (int k : kinds) {
     size_t smem = kernel_smem(k, a, c.tiles_per_block);
@@ -1882,7 +1885,15 @@ int pg_set_solver(pg_handle* h, int kind, int max_iter, double tolerance, int wa
   }
   if (warm_mode == PG_WARM_LEARNED && !h->mlp_loaded)
     return fail(PG_ERR_UNSUPPORTED, "no learned warm start is loaded (pg_set_warm_mlp)");
-  if (kind >= 0) h->dm.solver = kind;
+  if (kind >= 0 && kind != h->dm.solver) {
+    const int before = h->dm.solver;
+    h->dm.solver = kind;
+    CK(cudaSetDevice(h->device));
+    if (int rc = apply_cfg(h, h->cfg)) {  // the other solver's kernel in the same shapes
+      h->dm.solver = before;
+      return rc;
+    }
+  }
   if (max_iter >= 0) h->dm.iterations = max_iter;
   if (tolerance >= 0) h->dm.tolerance = tolerance;
   if (warm_mode >= 0) h->warm_mode = warm_mode;

@@ -220,3 +220,25 @@ def test_collision_lanes_by_pairs_and_batch():
                           (scenes.hull_tumble_xml(), 60, 16), (scenes.hull_tumble_xml(), 16 * sms + 1, 16)):
         with CudaPhysics(xml, n) as p:
             assert p.phase_launch()["collide"][0] == lanes, n
+
+
+def test_solver_switch_keeps_shapes_and_matches_a_model_compiled_for_it():
+    """PGS's kernel is prepared when a handle turns to it, at creation or by
+    pg_set_solver, in the shapes of the handle."""
+    n = 300
+    a = CudaPhysics(scenes.ant_xml(solver="PGS"), n)
+    b = CudaPhysics(scenes.ant_xml(), n)
+    b.set_launch(16, 8)
+    a.set_launch(16, 8)
+    b.set_solver(kind=1)
+    assert a.phase_launch() == b.phase_launch()
+    v = np.random.default_rng(1).normal(0, 1, (n, 14))
+    for p in (a, b):
+        p.set(Field.QVEL, range(n), v)
+        p.step(range(n), 40)
+    assert a.stats()["nrows"].any()
+    for f in Field:
+        np.testing.assert_array_equal(a.get(f, range(n)), b.get(f, range(n)))
+    b.set_solver(kind=0)
+    b.set_launch()
+    assert b.step_lanes() == 4

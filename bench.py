@@ -44,7 +44,8 @@ PHASE_STAGES = {"smooth": ("kinematics", "crba", "vel_rne", "passive_act", "fact
 # smooth 65.3 + 93.8 MB, collide 98.0 + 53.2 MB, Newton (newton_plain_kernel)
 # 131.7 + 48.6 MB per launch. The work record the phases hand each other (12 KB per env, 200 MB
 # at 16384 envs) is larger than the 126 MB L2, so most of it reaches HBM.
-NCU_TRAFFIC_PER_ENV = {"smooth": 9711.0, "collide": 9227.0, "newton": 11004.0}
+# The one-kernel step (quad_kernel, same batch and state): 15.4 + 73.4 MB.
+NCU_TRAFFIC_PER_ENV = {"smooth": 9711.0, "collide": 9227.0, "newton": 11004.0, "quad_kernel": 5424.0}
 # DRAM bytes (read + write) per image of render_kernel, from one ncu capture of a
 # whole frame of 4096 Ant images (the render benchmark's view): 8.2 + 274.0 MB
 # at 64 x 64, 6.8 + 787.6 MB at 128 x 128 (the images written are 12 B a pixel:
@@ -456,8 +457,8 @@ def run_ours(args):
                          "note": f"{top_flops:.0f} algorithmic FP64 ops per env in {top} (oracle "
                                  f"counters, {flops_step:.0f} per whole env-step) x {n} envs per launch / that "
                                  "kernel's mean event-timed duration (one kernel a substep: the step's); peak = live "
-                                 "DFMA microbenchmark (pg_fp64_peak); traffic = in-situ ncu DRAM bytes per env of a "
-                                 "phase kernel x envs",
+                                 "DFMA microbenchmark (pg_fp64_peak); traffic = in-situ ncu DRAM bytes per env of "
+                                 "that kernel x envs",
                          "hbm_achieved_gbs": bytes_step * n / (ms_ref / K * 1e-3) / 1e9},
             # the three phase kernels on the same states (PGS, the learned start and other models run them)
             "phases": {ph: {"ms_per_launch": phase_ms[ph] / K, "share": phase_ms[ph] / phase_total,

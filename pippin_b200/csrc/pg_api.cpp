@@ -416,6 +416,9 @@ struct Handle {
   int kind = STEP_PHASES;
   bool forced_shape = false;
   int* mixed = nullptr;
+  // one lane an env: the part of the blocks that its kernel reads, a column an
+  // env (LaneArgs), written with them
+  double* columns = nullptr;
   int warm_mode = WARM_REF_PREV_QACC;
   SubstepCfg cfg{{16, 4, 0}, {32, 4, 0}, {16, 4, 0}};
   int sm_count = 0;
@@ -759,6 +762,7 @@ LaneArgs lane_args(const Handle* h, int64_t count) {
   LaneArgs p{};
   p.t = h->lm;
   p.mixed = h->mixed;
+  p.columns = h->columns;
   p.sms = h->sm_count;
   // a full warp's worth of envs only once every SM sub-partition has a warp:
   // below that fewer envs a warp end the Newton loop sooner
@@ -1332,7 +1336,7 @@ void destroy(pg_handle* h) {
   cudaSetDevice(h->device);
   clear_graphs(h);
   void* ptrs[] = {h->d_model, h->qpos, h->qvel, h->ctrl, h->qacc, h->applied, h->params, h->iters, h->ncon,
-                  h->nrows, h->status, h->scratch, h->mixed, h->work, h->prev_con, h->prev_ncon, h->queue, h->order, h->b_ctrl.p, h->b_qout.p, h->b_poses_g.p,
+                  h->nrows, h->status, h->scratch, h->mixed, h->columns, h->work, h->prev_con, h->prev_ncon, h->queue, h->order, h->b_ctrl.p, h->b_qout.p, h->b_poses_g.p,
                   h->b_poses_c.p, h->b_dbg.p, h->b_vals.p, h->b_ids.p, h->learn.items, h->learn.feat, h->learn.force,
                   h->learn.rows, (void*)h->learn.mlp_w, (void*)h->learn.mlp_f, (void*)h->learn.mlp_err};
   for (void* p : ptrs)
@@ -1475,6 +1479,11 @@ int pg_create(const void* blob, size_t bytes, int64_t n_envs, int device, pg_han
   if (rc) return rc;
   rc = set_const_range(h.get(), 0, n_envs);
   if (rc) return rc;
+  if (h->kind == STEP_LANES && n_envs > 0) {
+    const size_t rows = h->dm.p_qpos_reset - h->dm.p_mass;
+    CK(cudaMalloc(&h->columns, sizeof(double) * rows * ((n + 31) / 32 * 32)));
+    CK(launch_columns(h->dm, h->params, n_envs, h->columns, h->stream));
+  }
   if (h->kind != STEP_PHASES && n_envs > 0) {
     // a launch of no substeps: the kernel's code and its lanes' local memory
     // are there before the first step (which must not allocate in
@@ -1738,8 +1747,8 @@ int pg_set_param(pg_handle* h, int param, int64_t id, int64_t start, int64_t end
   if ((rc = grow(h, h->b_vals, sizeof(double) * len))) return rc;
   const bool physical = param != PG_PARAM_GEOM_RGBA && param != PG_PARAM_QPOS0;
   CK(cudaMemcpyAsync(h->b_vals.p, values, sizeof(double) * len, cudaMemcpyHostToDevice, h->stream));
-  CK(launch_apply_param(h->dm, h->params + start * h->dm.pstride, end - start, param, id, (const double*)h->b_vals.p, w,
-                        m.nq, physical ? h->mixed : nullptr, h->stream));
+  CK(launch_apply_param(h->dm, h->params, start, end - start, param, id, (const double*)h->b_vals.p, w, m.nq,
+                        physical ? h->mixed : nullptr, h->columns, h->stream));
   if (param == PG_PARAM_BODY_MASS || param == PG_PARAM_BODY_INERTIA || param == PG_PARAM_BODY_IPOS) {
     if ((rc = set_const_range(h, start, end))) return rc;
   }

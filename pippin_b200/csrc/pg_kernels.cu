@@ -727,17 +727,48 @@ cudaError_t launch_substep(const StepArgs& a0, const SubstepCfg& c, cudaStream_t
   return cudaSuccess;
 }
 
-__global__ void apply_param_kernel(const __grid_constant__ DModel d, double* params, int64_t count, int p, int64_t id,
-                                   const double* v, int w, int nq, int* mixed) {
-  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (mixed && e == 0) *mixed = 1;
-  if (e < count) apply_param(d, params + e * d.pstride, p, id, v + e * w, nq);
+// entries [off, off + n) of env e's block into its column
+__device__ inline void fill_column(const DModel& d, const double* params, int64_t e, int off, int n, double* columns) {
+  double* c = columns + (e >> 5) * (int64_t)(d.p_qpos_reset - d.p_mass) * 32 + (e & 31);
+  for (int k = off; k < off + n; k++)
+    if (k >= d.p_mass && k < d.p_qpos_reset) c[(k - d.p_mass) * 32] = params[e * d.pstride + k];
 }
 
-cudaError_t launch_apply_param(const DModel& d, double* params, int64_t count, int p, int64_t id, const double* v, int w,
-                               int nq, int* mixed, cudaStream_t s) {
+__global__ void apply_param_kernel(const __grid_constant__ DModel d, double* params, int64_t start, int64_t count, int p,
+                                   int64_t id, const double* v, int w, int nq, int* mixed, double* columns) {
+  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (mixed && i == 0) *mixed = 1;
+  if (i >= count) return;
+  const int64_t e = start + i;
+  apply_param(d, params + e * d.pstride, p, id, v + i * w, nq);
+  if (!columns) return;
+  switch (p) {
+    case PG_PARAM_BODY_MASS:  // which rescales the inertia
+      fill_column(d, params, e, d.p_mass + (int)id, 1, columns);
+      [[fallthrough]];
+    case PG_PARAM_BODY_INERTIA: fill_column(d, params, e, d.p_inertia + 9 * (int)id, 9, columns); break;
+    case PG_PARAM_BODY_IPOS: fill_column(d, params, e, d.p_ipos + 3 * (int)id, 3, columns); break;
+    case PG_PARAM_DOF_DAMPING: fill_column(d, params, e, d.p_damping + (int)id, 1, columns); break;
+    case PG_PARAM_ACTUATOR_GAIN: fill_column(d, params, e, d.p_gain + (int)id, 1, columns); break;
+    case PG_PARAM_ACTUATOR_BIAS: fill_column(d, params, e, d.p_bias + 3 * (int)id, 3, columns); break;
+  }
+}
+
+cudaError_t launch_apply_param(const DModel& d, double* params, int64_t start, int64_t count, int p, int64_t id,
+                               const double* v, int w, int nq, int* mixed, double* columns, cudaStream_t s) {
   if (count <= 0) return cudaSuccess;
-  apply_param_kernel<<<(unsigned)((count + 127) / 128), 128, 0, s>>>(d, params, count, p, id, v, w, nq, mixed);
+  apply_param_kernel<<<(unsigned)((count + 127) / 128), 128, 0, s>>>(d, params, start, count, p, id, v, w, nq, mixed,
+                                                                     columns);
+  return cudaGetLastError();
+}
+
+__global__ void columns_kernel(const __grid_constant__ DModel d, const double* params, int64_t n, double* columns) {
+  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < n) fill_column(d, params, e, d.p_mass, d.p_qpos_reset - d.p_mass, columns);
+}
+cudaError_t launch_columns(const DModel& d, const double* params, int64_t n, double* columns, cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  columns_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(d, params, n, columns);
   return cudaGetLastError();
 }
 

@@ -39,10 +39,13 @@ cudaError_t launch_phase(int which, const StepArgs& a, const LaunchCfg& c, cudaS
 cudaError_t launch_set_const(const StepArgs& a, const LaunchCfg& c, const int* envs, int n, cudaStream_t s);
 cudaError_t launch_poses(const StepArgs& a, const LaunchCfg& c, float* geoms, float* cams, cudaStream_t s);
 cudaError_t launch_reset(const StepArgs& a, const int64_t* ids, int n, cudaStream_t s);
-// params[e * pstride ..] takes values v[e][w] of parameter p, element id, for
-// e < count; *mixed becomes 1 where it is given
-cudaError_t launch_apply_param(const DModel& d, double* params, int64_t count, int p, int64_t id, const double* v, int w,
-                               int nq, int* mixed, cudaStream_t s);
+// the parameter block of env e takes values v[e - start][w] of parameter p,
+// element id, for start <= e < start + count; *mixed becomes 1 where it is
+// given, and the env's column (LaneArgs) follows where there are columns
+cudaError_t launch_apply_param(const DModel& d, double* params, int64_t start, int64_t count, int p, int64_t id,
+                               const double* v, int w, int nq, int* mixed, double* columns, cudaStream_t s);
+// every env's column from its block
+cudaError_t launch_columns(const DModel& d, const double* params, int64_t n, double* columns, cudaStream_t s);
 // out[e][k] = params[e * pstride + off + k * step] for e < count, k < w
 cudaError_t launch_read_param(const double* params, int pstride, int64_t count, int off, int w, int step, double* out,
                               cudaStream_t s);

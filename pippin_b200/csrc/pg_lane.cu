@@ -67,7 +67,11 @@ __global__ void __launch_bounds__(32) lane_kernel(const __grid_constant__ StepAr
   const bool alive = lane < L;
   const int64_t item = item0 + (alive ? lane : L - 1);  // the others repeat the last env and write nothing
   const int64_t env = A.start + item;
-  const double* pp = A.st.params + (*P.mixed ? env * m.pstride : 0);
+  // env 0's block, or the env's column of its group's copy
+  const bool mixed = *P.mixed != 0;
+  const double* pp = mixed ? P.columns + (env >> 5) * (int64_t)(m.p_qpos_reset - m.p_mass) * 32 + (env & 31) - m.p_mass * 32
+                           : A.st.params;
+  const int ps = mixed ? 32 : 1;
   const double h = m.timestep;
 
   double q[LANE_NQ], v[N], f[N], qacc[N], hd[N];
@@ -81,7 +85,7 @@ __global__ void __launch_bounds__(32) lane_kernel(const __grid_constant__ StepAr
     const bool in = k < nv;
     v[k] = in ? A.st.qvel[env * nv + k] : 0.0;
     qacc[k] = in ? A.st.qacc[env * nv + k] : 0.0;
-    hd[k] = in ? pp[m.p_damping + k] : 0.0;
+    hd[k] = in ? pp[(m.p_damping + k) * ps] : 0.0;
     damped |= hd[k] != 0.0;
   }
   int status_all = P.sidx == 0 ? 0 : A.st.status[env];
@@ -180,7 +184,7 @@ __global__ void __launch_bounds__(32) lane_kernel(const __grid_constant__ StepAr
         }
         top++;
         path[top] = b;
-        walk_body(m, P.t, b, q, v, cdof, pp, s);
+        walk_body(m, P.t, b, q, v, cdof, pp, ps, s);
       }
     }
     // ------------------------------------------------ passive and actuator forces
@@ -205,8 +209,8 @@ __global__ void __launch_bounds__(32) lane_kernel(const __grid_constant__ StepAr
       double c = A.ctrl_seq ? A.ctrl_seq[((size_t)item * A.nstep + sidx) * nu + u] : A.st.ctrl[env * nu + u];
       if (A.ctrl_seq && alive) A.st.ctrl[env * nu + u] = c;  // rollout leaves the last controls in place
       if (m.act_ctrllimited[u]) c = clampd(c, m.act_ctrlrange[2 * u], m.act_ctrlrange[2 * u + 1]);
-      double fu = pp[m.p_gain + u] * c + pp[m.p_bias + 3 * u] + pp[m.p_bias + 3 * u + 1] * (gear * ls) +
-                  pp[m.p_bias + 3 * u + 2] * (gear * vs);
+      double fu = pp[(m.p_gain + u) * ps] * c + pp[(m.p_bias + 3 * u) * ps] + pp[(m.p_bias + 3 * u + 1) * ps] * (gear * ls) +
+                  pp[(m.p_bias + 3 * u + 2) * ps] * (gear * vs);
       if (m.act_forcelimited[u]) fu = clampd(fu, m.act_forcerange[2 * u], m.act_forcerange[2 * u + 1]);
       for (int k = a0; k < a0 + an; k++) f[m.jnt_dofadr[m.moment_jnt[k]]] += gear * m.moment_coef[k] * fu;
     }

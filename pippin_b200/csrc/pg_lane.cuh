@@ -51,9 +51,9 @@ __device__ __forceinline__ void walk_world(const DModel& m, Walk& s) {
 }
 // forward.rs:14-90, 115-164 for body b: on entry s holds its parent's pose,
 // velocity and acceleration, on return its own; its dofs' axes go to cdof.
-// q, v: the env's state; pp: its parameter block.
+// q, v: the env's state; pp, ps: its parameter block, the distance of its entries.
 __device__ __forceinline__ void walk_body(const DModel& m, const LaneModel& t, int b, const double* q, const double* v, double* cdof,
-                                          const double* pp, Walk& s) {
+                                          const double* pp, int ps, Walk& s) {
   V3& pos = s.pos;
   Q4& quat = s.quat;
   Sp &vel = s.vel, &acc = s.acc;
@@ -118,11 +118,11 @@ __device__ __forceinline__ void walk_body(const DModel& m, const LaneModel& t, i
     quat = unit(quat);
     xm = q_mat(quat);
   }
-  V3 ip{pp[m.p_ipos + 3 * b], pp[m.p_ipos + 3 * b + 1], pp[m.p_ipos + 3 * b + 2]};
+  V3 ip{pp[(m.p_ipos + 3 * b) * ps], pp[(m.p_ipos + 3 * b + 1) * ps], pp[(m.p_ipos + 3 * b + 2) * ps]};
   M3 in;
 #pragma unroll
-  for (int t = 0; t < 9; t++) in.m[t] = pp[m.p_inertia + 9 * b + t];
-  double mass = pp[m.p_mass + b];
+  for (int t = 0; t < 9; t++) in.m[t] = pp[(m.p_inertia + 9 * b + t) * ps];
+  double mass = pp[(m.p_mass + b) * ps];
   // R I R' + m (|c|^2 1 - c c'), upper triangle
   V3 c = pos + mv(xm, ip);
   M3 ri = mm(xm, in);

@@ -46,6 +46,9 @@ struct LaneArgs {
   // pg_set_param has written one. Read when the kernel runs, so that a
   // captured step replays with the parameters of that time.
   const int* mixed;
+  // the blocks' entries from p_mass up to p_qpos_reset, a column an env, in
+  // groups of 32: what a lane reads together lies together (one lane an env)
+  const double* columns;
   int lanes;           // envs a warp takes (1..32)
   int sms;             // SMs of the GPU
   int sidx, nsub;      // substeps [sidx, sidx + nsub) of the call

@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(32 * QUAD_WARPS, 1) quad_kernel(const __grid_c
           if (l0 == 0 && k == 0 && P.t.limb_n > 4) end = s;
           if (k < 0 || a0 + k < a1) {
             int b = k < 0 ? P.t.trunk[P.t.trunk_n + k] : P.t.limb_body[a0 + k];
-            walk_body(m, P.t, b, q, v, cdof, pp, s);
+            walk_body(m, P.t, b, q, v, cdof, pp, 1, s);
             if (k < 0) geoms(b, r, 4, s);
             else geoms(b, 0, 1, s);
             keep(k < 0 ? tr + 16 * (P.t.trunk_n + k) : lb + 16 * k, s.I, s.fr);

@@ -242,3 +242,42 @@ def test_solver_switch_keeps_shapes_and_matches_a_model_compiled_for_it():
     b.set_solver(kind=0)
     b.set_launch()
     assert b.step_lanes() == 4
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 100])
+def test_one_lane_columns_follow_every_parameter(n):
+    """The one-lane kernel reads per-env parameters from columns written with
+    the blocks: each parameter it uses, for a part of the envs, against a
+    handle on the phase kernels."""
+    m = mjcf.load_string(scenes.arm3d_xml())
+    blob = mjcf.to_blob(m)
+    a, b = CudaPhysics(blob, n), CudaPhysics(blob, n)
+    b.set_launch(16, 4)
+    assert (a.step_lanes(), b.step_lanes()) == (1, 0)
+    rng = np.random.default_rng(n)
+    q, v = _states(m, n, rng)
+    ctrl = rng.uniform(-1, 1, (n, m.nu))
+    base = None
+    for pid, elem in ((None, 0), (Param.BODY_MASS, 2), (Param.BODY_INERTIA, m.nbody - 1), (Param.BODY_IPOS, 3),
+                      (Param.DOF_DAMPING, 4), (Param.ACTUATOR_GAIN, 1), (Param.ACTUATOR_BIAS, 2), (Param.GEOM_SIZE, 1),
+                      (Param.GEOM_FRICTION, 1), (Param.BODY_MASS, 1)):
+        s0 = n // 3
+        if pid is not None:
+            w = a.param_width(pid)
+            val = a.get_param(pid, elem, range(s0, n)) + rng.uniform(0.1, 0.5, (n - s0, w)) * (
+                0.01 if pid in (Param.BODY_INERTIA, Param.BODY_IPOS) else 1.0)
+            for p in (a, b):
+                p.set_param(pid, elem, range(s0, n), val)
+        for p in (a, b):
+            p.set(Field.QPOS, range(n), q)
+            p.set(Field.QVEL, range(n), v)
+            p.set(Field.CTRL, range(n), ctrl)
+            p.step(range(n), 1)
+        qa, qb = a.get(Field.QACC, range(n)), b.get(Field.QACC, range(n))
+        assert _rel(qa, qb) < TOL, pid
+        if pid is None:
+            base = qa
+        else:
+            np.testing.assert_array_equal(qa[:s0], base[:s0])
+        if pid == Param.BODY_MASS:
+            assert _rel(qa[s0:], base[s0:]) > 1e-4

@@ -665,7 +665,8 @@ int choose_grid(Handle* h, int phase, const LaunchCfg& want, LaunchCfg* out) {
   std::vector<int> kinds = {phase};
   if (phase == K_SMOOTH) kinds = {K_SMOOTH, K_SET_CONST, K_POSES};
   if (phase == K_NEWTON) {
-    kinds = {K_NEWTON, K_NEWTON_PLAIN};  // with and without the learned start's code
+    // with and without the learned start's code
+    kinds = {K_NEWTON, h->dm.nblock > 1 ? K_NEWTON_ISLANDS : K_NEWTON_PLAIN};
     if (h->dm.solver == SOLVER_PGS) kinds.push_back(K_PGS);  // (its code loads with the first handle that steps PGS)
   }
   int per_sm = 0;

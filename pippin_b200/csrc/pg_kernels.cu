@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(256, 2) collide_kernel(const __grid_constant__
 // lanes an SM, one wave for 4096 Ant envs. LEARN = false (newton_plain_kernel,
 // launched when the learned start neither predicts nor collects) leaves the
 // learned start's code out of the kernel.
-template <int G, bool LEARN, bool PGS>
+template <int G, bool LEARN, bool PGS, bool ONE>
 __device__ __forceinline__ void newton_phase(const StepArgs& A) {
   extern __shared__ __align__(16) unsigned char smem[];
   const DModel& m = stage_model(A, smem);
@@ -300,7 +300,7 @@ __device__ __forceinline__ void newton_phase(const StepArgs& A) {
             if (A.learn.mode == LEARN_DUMP) ldump = A.learn.rows + (size_t)lbase * 4;
           }
         }
-        iters = newton_solve<G, LEARN>(T, m, w, A.s, e, nr, acc, warm, lfeat, lforce, lnum, ldump);
+        iters = newton_solve<G, LEARN, ONE>(T, m, w, A.s, e, nr, acc, warm, lfeat, lforce, lnum, ldump);
         if (wk[A.k.meta + K_META_DAMPED] != 0.0) {
           const double* lh = w.fac >= 0 ? ws + w.fac : wk + A.k.lh;
           if (w.fac >= 0) load_async(T, ws + w.fac, wk + A.k.lh, nv * nv);
@@ -337,17 +337,28 @@ __device__ __forceinline__ void newton_phase(const StepArgs& A) {
 
 template <int G>
 __global__ void __launch_bounds__(256, 2) newton_kernel(const __grid_constant__ StepArgs A) {
-  newton_phase<G, true, false>(A);
+  newton_phase<G, true, false, false>(A);
 }
 template <int G>
 __global__ void __launch_bounds__(256, 2) newton_plain_kernel(const __grid_constant__ StepArgs A) {
-  newton_phase<G, false, false>(A);
+  newton_phase<G, false, false, true>(A);
 }
-// (in a kernel of its own: with both solvers in one, each solver's loops
-// spilled more)
+// Several trees, and PGS, in kernels of their own: the register Newton spills
+// more the more code stands beside it (Newton phase of 16384 Ant envs 290 us
+// with islands on the tile in the same kernel, 315 with islands on lanes and
+// both kinds of PGS, 262 alone). On 32 lanes the islands' lanes take 168
+// registers, since shared memory holds a block to 128 threads and an SM to 384
+// (4096 envs of hulls 754 -> 675 us; newton_tree's spilled loads 1016 -> 472
+// bytes). The one tree's code stays in here: without it the compiler spilled
+// more in the rest (hulls 754 against 724 at 128 registers).
+template <int G>
+__global__ void __launch_bounds__(G == 32 ? 384 : 256, G == 32 ? 1 : 2)
+    newton_islands_kernel(const __grid_constant__ StepArgs A) {
+  newton_phase<G, false, false, false>(A);
+}
 template <int G>
 __global__ void __launch_bounds__(256, 2) pgs_kernel(const __grid_constant__ StepArgs A) {
-  newton_phase<G, false, true>(A);
+  newton_phase<G, false, true, false>(A);
 }
 
 // whether a substep's Newton phase needs the learned start's code
@@ -652,6 +663,7 @@ static const void* kernel_ptr(int which) {
     case K_COLLIDE: return (const void*)collide_kernel<G>;
     case K_NEWTON: return (const void*)newton_kernel<G>;
     case K_NEWTON_PLAIN: return (const void*)newton_plain_kernel<G>;
+    case K_NEWTON_ISLANDS: return (const void*)newton_islands_kernel<G>;
     case K_PGS: return (const void*)pgs_kernel<G>;
     case K_SET_CONST: return (const void*)set_const_kernel<G>;
     case K_POSES: return (const void*)poses_kernel<G>;
@@ -676,6 +688,7 @@ size_t kernel_smem(int which, const StepArgs& a, int tiles_per_block) {
                           (collide_tile_ints(a.m) * sizeof(int) + collide_cache_doubles(a.m) * sizeof(double));
     case K_NEWTON:
     case K_NEWTON_PLAIN:
+    case K_NEWTON_ISLANDS:
     case K_PGS: return staged + (size_t)tiles_per_block * a.wn.stride * sizeof(double);
     default: return staged + (size_t)tiles_per_block * a.w.stride * sizeof(double);
   }
@@ -723,6 +736,7 @@ cudaError_t launch_substep(const StepArgs& a0, const SubstepCfg& c, cudaStream_t
   }
   if (a.m.solver == SOLVER_PGS) PG_LAUNCH(K_PGS, pgs_kernel, c.newton, a);
   else if (newton_learns(a)) PG_LAUNCH(K_NEWTON, newton_kernel, c.newton, a);
+  else if (a.m.nblock > 1) PG_LAUNCH(K_NEWTON_ISLANDS, newton_islands_kernel, c.newton, a);
   else PG_LAUNCH(K_NEWTON_PLAIN, newton_plain_kernel, c.newton, a);
   return cudaSuccess;
 }
@@ -822,6 +836,7 @@ cudaError_t launch_phase(int which, const StepArgs& a0, const LaunchCfg& c, cuda
     case K_NEWTON:
       if (a.m.solver == SOLVER_PGS) PG_LAUNCH(K_PGS, pgs_kernel, c, a);
       else if (newton_learns(a)) PG_LAUNCH(K_NEWTON, newton_kernel, c, a);
+      else if (a.m.nblock > 1) PG_LAUNCH(K_NEWTON_ISLANDS, newton_islands_kernel, c, a);
       else PG_LAUNCH(K_NEWTON_PLAIN, newton_plain_kernel, c, a);
       break;
     default: return cudaErrorInvalidValue;

@@ -7,7 +7,8 @@
 namespace pg {
 
 // tile kernels (one env per tile of G lanes, persistent over a work counter)
-enum { K_SMOOTH = 0, K_COLLIDE = 1, K_NEWTON = 2, K_SET_CONST = 3, K_POSES = 4, K_NEWTON_PLAIN = 5, K_PGS = 6, K_COUNT = 7 };
+enum { K_SMOOTH = 0, K_COLLIDE = 1, K_NEWTON = 2, K_SET_CONST = 3, K_POSES = 4, K_NEWTON_PLAIN = 5, K_PGS = 6,
+       K_NEWTON_ISLANDS = 7, K_COUNT = 8 };
 
 struct LaunchCfg {
   int G;                // lanes per environment (8, 16, 32)

@@ -1306,8 +1306,9 @@ __device__ void dump_row_forces(const Tile<G>& T, int nv, const double* J, const
 }
 
 // newton.rs:378-473. LEARN = false compiles the learned start's inputs out
-// (a kernel for the other warm-start modes carries none of its code).
-template <int G, bool LEARN = true>
+// (a kernel for the other warm-start modes carries none of its code), ONE the
+// islands'.
+template <int G, bool LEARN, bool ONE>
 __device__ int newton_solve(const Tile<G>& T, const DModel& m, const WsLayout& w, const ScrLayout& s,
                             const EnvCtx& e, int nr, double* a, const double* warm, const float* lfeat = nullptr,
                             const float* lforce = nullptr, int lnum = 0, float* ldump = nullptr) {
@@ -1345,10 +1346,12 @@ __device__ int newton_solve(const Tile<G>& T, const DModel& m, const WsLayout& w
   }
   T.sync();
   NewtonBufs B{ws + w.a0, ws + w.grad, ws + w.p, ws + w.tmp, ws + w.tmp2, ws + w.mp, e.fac, ws + w.rinv};
-  if (m.nblock > 1) {
-    int it = newton_islands<G, !LEARN>(T, m, w, s, e, nr, a, warm, B, cand);
-    if (learned && ldump) dump_row_forces(T, nv, J, R, a, 4 * lnum, ldump);
-    return it;
+  if constexpr (!ONE) {
+    if (m.nblock > 1) {
+      int it = newton_islands<G, !LEARN>(T, m, w, s, e, nr, a, warm, B, cand);
+      if (learned && ldump) dump_row_forces(T, nv, J, R, a, 4 * lnum, ldump);
+      return it;
+    }
   }
   // one tree: the rows either touch it (one island spanning everything)
   // or none has a nonzero entry (no island: nothing is solved)

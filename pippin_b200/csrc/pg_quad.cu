@@ -4,8 +4,8 @@
 //
 // The three phase kernels' tiles of 16 lanes leave three lanes in four idle
 // on the tree walks, hand 12 KB an env through HBM and take 10,600 warp
-// instructions an Ant env-step. Here eight envs share a warp (2,500
-// instructions an env-step) and nothing leaves the SM but the contacts:
+// instructions an Ant env-step. Here eight envs share a warp (2,500 to 4,850
+// instructions an env-step, by the contacts) and nothing leaves the SM but the contacts:
 //   - every lane walks the trunk, then a limb of its own, in registers;
 //   - M, the dof axes and one contact's Jacobian sit in shared memory (2.3 KB
 //     an env), rows of the matrix being factored in registers, cyclic over
@@ -25,8 +25,8 @@
 // staged in shared memory was slower than read through L1 (1260 against 1194).
 //
 // Measured (B200, Ant, us a call with three batches in flight; phase kernels
-// before): 16384 envs, one substep 732 -> 336; 65536 envs 2502 -> 1187; 4096
-// envs, four substeps, host buffers 905 -> 646; 16 envs 175 -> 156.
+// before): 16384 envs, one substep 732 -> 334; 65536 envs 2502 -> 1182; 4096
+// envs, four substeps, host buffers 905 -> 641; 16 envs 175 -> 152.
 #include <cuda_runtime.h>
 
 #include <algorithm>

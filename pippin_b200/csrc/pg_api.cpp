@@ -738,9 +738,10 @@ int set_const_range(Handle* h, int64_t start, int64_t end) {
 //   13 / 13 / 13 against 45 / 45 / 52 / 118, cartpole 17 / 20 / 21 / 21 against
 //   56 / 54 / 63 / 163. Past 8 dofs a lane's matrix spills: two arms of 15
 //   dofs 86 / 141 / 140 / 143 (1 / 512 / 4096 / 16384 envs, with the wait)
-//   against 83 / 83 / 160 / 402; four lanes 74 / 76 / 77 / 158. With rows a lane's Newton loses to the phase kernels in the
-//   middle of the range (a 6-hinge chain: 62 / 145 / 200 / 259 against 94 /
-//   130 / 167 / 446), so such models go elsewhere;
+//   against 83 / 83 / 160 / 402; four lanes 74 / 76 / 77 / 158. With rows a
+//   lane's Newton loses to the phase kernels in the middle of the range (a
+//   6-hinge chain: 62 / 145 / 200 / 259 against 94 / 130 / 167 / 446), so such
+//   models go elsewhere;
 //   four lanes, one tree with rows possible: Ant 65 / 95 / 113 / 217 against
 //   103 / 129 / 166 / 541, three limbs of 12 dofs 65 / 129 / 168 / 311 against
 //   110 / 161 / 257 / 653, five limbs of 16 dofs 78 / 181 / 244 / 509 against
@@ -772,7 +773,7 @@ LaneArgs lane_args(const Handle* h, int64_t count) {
   while (p.lanes < most && count > (int64_t)p.lanes * 4 * h->sm_count) p.lanes *= 2;
   return p;
 }
-// nstep substeps of [start, end) one lane per env, LANE_CHUNK a launch
+// nstep substeps of [start, end) on one or four lanes an env, LANE_CHUNK a launch
 constexpr int64_t LANE_CHUNK = 64;
 int enqueue_lanes(Handle* h, StepArgs a, int64_t start, int64_t end, int64_t nstep) {
   a.start = (int)start;

@@ -5,14 +5,14 @@
 // A tile of 16 lanes leaves most of them idle on such trees (a chain has one
 // body a level) and pays every instruction per env; here 32 envs share each
 // one. 16384 cartpoles took 2927 warp instructions an env and substep, now
-// 140. A call's substeps run in one launch with the state in registers and
+// 104. A call's substeps run in one launch with the state in registers and
 // local arrays, so ten substeps read and write it once. M is factored last
 // row first (H = L' D L) in registers with the compile-time size N, every
 // index constant: rolled loops over a local array made each entry a round
 // trip to L1 (50k cycles a factor of 14 rows against 6k).
 //
 // Measured (B200, 16384 envs, ten substeps a call): cartpole 1620 us with the
-// phase kernels, 155 us; with three batches in flight 1398 against 72 us a
+// phase kernels, 110 us; with three batches in flight 1398 against 53 us a
 // batch. What bounds it: dependent FP64 instructions of one warp a
 // sub-partition (about 5 cycles each) up to some 20,000 envs.
 #include <cuda_runtime.h>

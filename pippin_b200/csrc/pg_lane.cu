@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(32) lane_kernel(const __grid_constant__ StepAr
   const int64_t item = item0 + (alive ? lane : L - 1);  // the others repeat the last env and write nothing
   const int64_t env = A.start + item;
   // env 0's block, or the env's column of its group's copy
-  const bool mixed = *P.mixed != 0;
+  const bool mixed = __any_sync(FULL, *P.mixed != 0);  // (the same for the warp: uniform to the compiler too)
   const double* pp = mixed ? P.columns + (env >> 5) * (int64_t)(m.p_qpos_reset - m.p_mass) * 32 + (env & 31) - m.p_mass * 32
                            : A.st.params;
   const int ps = mixed ? 32 : 1;
